@@ -188,3 +188,65 @@ def tolerance(case):
     # Two correct fp32 evaluations of the gate/up contraction differ in the last bits, so a
     # few of the bf16 intermediates land on the neighbouring value.
     return {"rel": 2e-4, "differ": 2e-4}
+
+
+_E2M1 = (0.0, 0.5, 1.0, 1.5, 2.0, 3.0, 4.0, 6.0, -0.0, -0.5, -1.0, -1.5, -2.0, -3.0, -4.0, -6.0)
+
+
+def _dequant64(blocks, scales):
+    """[rows, G, 16] e2m1 pairs (even column in the low half) and [rows, G] e8m0 bytes -> [rows, 32 G]."""
+    table = torch.tensor(_E2M1, dtype=torch.float64, device=blocks.device)
+    v = torch.stack((table[(blocks & 15).long()], table[(blocks >> 4).long()]), dim=-1).flatten(-2)
+    return (v * torch.exp2(scales.double() - 127.0).unsqueeze(-1)).flatten(-2)
+
+
+def exact(case, seed):
+    """What run() returns, in 64 bits.  The two roundings to bf16 that the block's contract
+    names (its input, and the SwiGLU output in front of the down projection) are part of the
+    result; everything between them is not rounded."""
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(1000 + seed)
+    H, I, E, K, L, T = (case[k] for k in ("H", "I", "E", "K", "layers", "tokens"))
+    if case["op"] == "unpack":
+        return None  # bytes, compared as they are
+
+    def randn(*shape):
+        return torch.randn(*shape, generator=gen, device="cuda")
+
+    layers = []
+    for layer in range(L):
+        zipf = dict(zipf_s=1.1, zipf_gain=synth.ZIPF_GAIN_4X) if case["zipf"] else {}
+        wr, br = synth.make_router(_shape(case), seed=seed * 64 + layer, **zipf)
+        router = (torch.from_numpy(synth.bf16_bits_to_f32(wr)).cuda().double(), torch.from_numpy(br).cuda().double())
+        layers.append((router, (_random_bytes((E, 2 * I, H // 32, 16), gen), _scales((E, 2 * I, H // 32), gen),
+                                0.01 * randn(E, 2 * I), _random_bytes((E, H, I // 32, 16), gen),
+                                _scales((E, H, I // 32), gen), 0.01 * randn(E, H))))
+    x = randn(L, T, H)
+    if case["op"] == "norm":
+        w = 1.0 + 0.1 * randn(L, H)
+        w = w.to(torch.bfloat16) if case["dtype"] == "bf16" else w
+    elif case["dtype"] == "f32":
+        x = randn(L, T, H)
+
+    out, side = [], []
+    for layer, ((wr, br), (b1, s1, c1, b2, s2, c2)) in enumerate(layers):
+        t = x[layer].double()
+        if case["op"] == "norm":
+            t = w[layer].double() * (t / torch.sqrt((t * t).mean(dim=-1, keepdim=True) + 1e-5))
+        t = t.float().to(torch.bfloat16).double()
+        scores = t @ wr.T + br
+        top, index = scores.topk(K, dim=-1)
+        weight = torch.softmax(top, dim=-1)
+        y = x[layer].double() if case["op"] == "norm" else torch.zeros(T, H, dtype=torch.float64, device="cuda")
+        for e in index.unique().tolist():
+            rows, k = (index == e).nonzero(as_tuple=True)
+            g = t[rows] @ _dequant64(b1[e], s1[e]).T + c1[e].double()
+            gate, up = g[:, 0::2].clamp(max=7.0), g[:, 1::2].clamp(-7.0, 7.0)
+            h = (gate * torch.sigmoid(1.702 * gate) * (up + 1.0)).to(torch.bfloat16).double()
+            y[rows] += weight[rows, k].unsqueeze(-1) * (h @ _dequant64(b2[e], s2[e]).T + c2[e].double())
+        out.append(y)
+        side.append((scores, None, weight))
+    if case["op"] == "host":
+        return (out[0], None, side[0][2]) if case["side"] else out[0]
+    out = torch.stack(out)
+    return (out, side) if case["side"] else out
