@@ -144,26 +144,6 @@ __host__ __device__ __forceinline__ uint32_t mxfp4_retile_word(uint32_t w) {
     return r;
 }
 
-// Exact decode of one element for ANY scale byte, integer arithmetic only:
-// the bf16 bit pattern of LUT[code] * 2^(scale_byte-127) as the reference's
-// dequantize_fp4 produces it
-// (tools/model_export/gpt-oss-20b/export_model_bin.py:75-133), including the
-// bf16 subnormals at scale byte 0 and the overflow to inf at 254/255.
-__host__ __device__ __forceinline__ uint32_t mxfp4_decode_exact(uint32_t code, uint32_t scale_byte) {
-    uint32_t sign = (code & 8u) << 12;
-    uint32_t m = code & 7u;
-    if (m == 0)
-        return sign;
-    uint32_t mant = (m >= 2) ? (m & 1u) : 0u;
-    int biased = (int)scale_byte + ((m >= 2) ? (int)(m >> 1) - 1 : -1);
-    if (biased >= 255)
-        return sign | 0x7F80u;
-    if (biased >= 1)
-        return sign | ((uint32_t)biased << 7) | (mant << 6);
-    // subnormal result: (2 + mant) * 2^(biased - 128), unit 2^-133
-    return sign | ((2u + mant) << (biased + 5));
-}
-
 __host__ __device__ __forceinline__ int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // Programmatic dependent launch.  A kernel launched with the programmatic-serialization

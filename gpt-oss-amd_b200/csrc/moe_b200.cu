@@ -1418,16 +1418,15 @@ moe_b200_status moe_b200_mxfp4_unpack(const uint8_t* blocks, const uint8_t* scal
     const long long n_blocks = rows * G;
     if (n_blocks == 0)
         return MOE_B200_OK;
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
         cudaGetLastError();
         return fail(nullptr, MOE_B200_ERR_NO_DEVICE, "no CUDA device; this library has no CPU path");
     }
-    long long want = (n_blocks + 255) / 256;
-    int grid = (int)(want < (long long)sms * 8 ? want : (long long)sms * 8);
-    mxfp4_unpack_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(blocks, scales,
-                                                                                   n_blocks, out_bf16);
+    const long long n_words = n_blocks * 4, per_block = UNPACK_THREADS * UNPACK_WORDS;
+    const long long grid = (n_words + per_block - 1) / per_block;
+    mxfp4_unpack_kernel<<<(unsigned)grid, UNPACK_THREADS, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        reinterpret_cast<const uint32_t*>(blocks), scales, n_words, reinterpret_cast<uint4*>(out_bf16));
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return fail(nullptr, MOE_B200_ERR_CUDA, cudaGetErrorString(e));
