@@ -26,7 +26,9 @@
 // cycles), shared memory carries only the packed bytes and the small activation tile.
 //
 // One persistent CTA per SM walks work items (expert, 128-row weight tile, tile
-// of up to 64 token rows).  A pipeline STEP covers CS = 6 chunks of 64 K-columns
+// of up to 64 token rows, or 128 in the wide variant: medium batches, where 64-row items
+// would decode most weights twice and CTA pairs run half-empty tiles; figures at Narrow and
+// Wide below).  A pipeline STEP of the narrow form covers CS = 6 chunks of 64 K-columns
 // (384 columns, 26 KB of packed weights: one bulk copy, the chunks of a weight
 // tile are contiguous).  Two measurements set that size.  (1) Bulk copies of one
 // chunk (4352 B) stream at 2.6 TB/s over the whole GPU however deep the ring is,
@@ -65,34 +67,48 @@ namespace tc5 {
 namespace ts {
 
 constexpr int BN = 64;                       // most token rows per work item (UMMA N)
-constexpr int CS = STEP_CHUNKS;              // chunks of 64 K-columns per pipeline step
-constexpr int B_UNIT_BYTES = CS * 32 * 128;  // activation tiles of one step for 32 token rows (32 rows x 64 bf16 per chunk, SW128)
-constexpr int SBU = 4;                       // units in the B ring
-constexpr int W_SLOT_BYTES = CS * CHUNK_BYTES;
+constexpr int BN_WIDE = 128;                 // the same of the wide variant
 constexpr int A_SUB_COLS = KSTAGE / 2;       // one decoded chunk in tensor memory: 128 lanes x 32 columns of bf16x2
-constexpr int A_SLOT_COLS = CS * A_SUB_COLS;
 constexpr int MMA_WARP = 2;
 constexpr int DEQ_WARP0 = 3;
 constexpr int G = 2;                         // decode groups
 constexpr int GW = 8;                        // warps per decode group: two per quarter of the rows
-//   SA  A slots (tensor memory)   SB  activation slots   WS  packed slots   NB  barrier pairs
-// SA and WS are multiples of G, so the successive fills of a slot are handled by one
-// group in program order (an mbarrier parity wait cannot tell phase n from phase n-2).
-constexpr int SA = 2, NB = 4, WS = 4;
 constexpr int SETS = 2;                      // accumulator sets: the MMAs of item i+1 overlap the epilogue of item i
-constexpr int TMEM_A0 = SETS * BN;           // first tensor-memory column of the A slots
 constexpr int TMEM_COLS = 512;
-static_assert(TMEM_A0 + SA * A_SLOT_COLS <= TMEM_COLS, "tensor memory");
-static_assert(SA % G == 0 && WS % G == 0 && NB % SA == 0 && NB % G == 0 && NB >= SBU,
-              "a slot's successive fills must belong to one decode group");
 constexpr int EPI_WARP0 = DEQ_WARP0 + GW * G;
 constexpr int N_THREADS = (EPI_WARP0 + 4) * 32;  // 736
 constexpr int MAX_LOCAL_EXPERTS = 256;
 constexpr int EPI_STAGE_BYTES = 2048;
-constexpr int N_BARRIERS = 2 * WS + 2 * NB + 2 * SETS;
-constexpr int SMEM_BYTES = SBU * B_UNIT_BYTES + WS * W_SLOT_BYTES + 4 * EPI_STAGE_BYTES + N_BARRIERS * 8 +
-                           (MAX_LOCAL_EXPERTS + 1) * 3 * 4 + 64 + 1024;
-static_assert(SMEM_BYTES <= 227 * 1024, "shared memory per CTA");
+
+//   BN  most token rows of an item    CS  chunks of 64 K-columns per pipeline step
+//   SA  A slots (tensor memory)       SB  B slots (units of 32 rows where the item decides how
+//   WS  packed slots                      many it takes, BN rows where UNITS is false)
+// NB barrier pairs.  SA and WS are multiples of G, so the successive fills of a slot are handled
+// by one group in program order (an mbarrier parity wait cannot tell phase n from phase n-2).
+template <int BN_, int CS_, int SA_, int SB_, int WS_, int NB_, bool UNITS_>
+struct Config {
+    static constexpr int BN = BN_, CS = CS_, SA = SA_, SB = SB_, WS = WS_, NB = NB_;
+    static constexpr bool UNITS = UNITS_;
+    static constexpr int B_SLOT_BYTES = CS * (UNITS ? 32 : BN) * 128;  // rows x 64 bf16 per chunk, SW128
+    static constexpr int W_SLOT_BYTES = CS * CHUNK_BYTES;
+    static constexpr int A_SLOT_COLS = CS * A_SUB_COLS;
+    static constexpr int TMEM_A0 = SETS * BN;  // first tensor-memory column of the A slots
+    static constexpr int N_BARRIERS = 2 * WS + 2 * NB + 2 * SETS;
+    static constexpr int SMEM_BYTES = SB * B_SLOT_BYTES + WS * W_SLOT_BYTES + 4 * EPI_STAGE_BYTES + N_BARRIERS * 8 +
+                                      (MAX_LOCAL_EXPERTS + 1) * 3 * 4 + 64 + 1024;
+    static_assert(TMEM_A0 + SA * A_SLOT_COLS <= TMEM_COLS, "tensor memory");
+    static_assert(SA % G == 0 && WS % G == 0 && NB % SA == 0 && NB % G == 0 && NB >= SB,
+                  "a slot's successive fills must belong to one decode group");
+    static_assert(SMEM_BYTES <= 227 * 1024, "shared memory per CTA");
+};
+// Up to 64 rows per item: six chunks per step.  (Three chunks with four A slots, and three
+// decode warps per quarter instead of two, measured again on this form: 256 tokens, 32
+// experts 157 us per layer; 181 with three chunks, 167 with three warps.)
+using Narrow = Config<BN, STEP_CHUNKS, 2, 4, 4, 4, true>;
+// Up to 128 rows: a weight tile is decoded once for twice the rows.  Accumulators and B
+// tiles double, so a step has three chunks.  (Two chunks with four A slots: 777 tokens 285 us
+// instead of 258; four chunks with two B slots: 265.)
+using Wide = Config<BN_WIDE, 3, 2, 3, 4, 4, false>;
 
 // D[tmem] (+)= A[tmem] . B[smem desc]^T: A is 128 lanes x 8 columns (16 bf16 of K per lane).
 // The shared-memory descriptor comes as its two 32-bit halves: stepping through a tile
@@ -118,8 +134,9 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t a[3
           "r"(a[16]), "r"(a[17]), "r"(a[18]), "r"(a[19]), "r"(a[20]), "r"(a[21]), "r"(a[22]), "r"(a[23]),
           "r"(a[24]), "r"(a[25]), "r"(a[26]), "r"(a[27]), "r"(a[28]), "r"(a[29]), "r"(a[30]), "r"(a[31])
         : "memory");
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
+// All of this thread's tensor-memory stores are done.
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 struct TileInfo {
     int e;        // local expert
@@ -138,6 +155,7 @@ struct TileTables {
 
 // Items ordered [expert][weight tile][token tile]: the token tiles that share
 // packed weights run on neighbouring CTAs at the same time and meet in L2.
+template <class C>
 __device__ __forceinline__ TileInfo decode_tile(int tile, int m_tiles, const TileTables& tt, int E) {
     int lo = 0, hi = E;
     while (hi - lo > 1) {
@@ -152,17 +170,25 @@ __device__ __forceinline__ TileInfo decode_tile(int tile, int m_tiles, const Til
     const int ntl = tt.tile_start[lo + 1] - tt.tile_start[lo];
     const int r = tile - tt.tile_start[lo] * m_tiles;
     ti.mt = r / ntl;
-    const int n0 = (r - ti.mt * ntl) * BN;
+    const int cnt = tt.cnt[lo];
+    int rows = C::BN;
+    if (!C::UNITS && ntl > 1) {
+        // items of equal size: the weights are decoded once per item whatever its rows
+        const int q = ((cnt + ntl - 1) / ntl + 31) & ~31;
+        if ((ntl - 1) * q < cnt)
+            rows = q;
+    }
+    const int n0 = (r - ti.mt * ntl) * rows;
     ti.row0 = tt.off[lo] + n0;
-    ti.valid_n = min(BN, tt.cnt[lo] - n0);
+    ti.valid_n = min(rows, cnt - n0);
     ti.n_mma = max(32, (ti.valid_n + 31) & ~31);
-    ti.box_idx = ti.n_mma <= 32 ? 0 : 1;
+    ti.box_idx = ti.n_mma <= 32 ? 0 : ti.n_mma <= 64 ? 1 : 2;
     return ti;
 }
 
 // m_tiles: 128-row weight tiles per expert matrix (rows padded to 128 in the resident
 // layout); out_rows_valid: features (MODE 0) or output columns (MODE 1) that exist.
-template <int MODE>
+template <int MODE, class C>
 __global__ void __launch_bounds__(N_THREADS, 1)
 expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __restrict__ chunks,
                       size_t expert_stride, int k_stages, int m_tiles,
@@ -178,30 +204,30 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
     unsigned char* smem = reinterpret_cast<unsigned char*>(
         (reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~(uintptr_t)1023);
     unsigned char* b_ring = smem;
-    unsigned char* w_ring = b_ring + SBU * B_UNIT_BYTES;
-    unsigned char* epi_stage = w_ring + WS * W_SLOT_BYTES;
+    unsigned char* w_ring = b_ring + C::SB * C::B_SLOT_BYTES;
+    unsigned char* epi_stage = w_ring + C::WS * C::W_SLOT_BYTES;
     uint64_t* bars = reinterpret_cast<uint64_t*>(epi_stage + 4 * EPI_STAGE_BYTES);
-    int* s_tables = reinterpret_cast<int*>(bars + N_BARRIERS);
+    int* s_tables = reinterpret_cast<int*>(bars + C::N_BARRIERS);
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(s_tables + 3 * (MAX_LOCAL_EXPERTS + 1));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
     const uint32_t bar0 = smem_u32(bars);
     auto bar_w_full = [&](int s) { return bar0 + 8u * (uint32_t)s; };
-    auto bar_w_empty = [&](int s) { return bar0 + 8u * (uint32_t)(WS + s); };
-    auto bar_full = [&](int s) { return bar0 + 8u * (uint32_t)(2 * WS + s); };
-    auto bar_empty = [&](int s) { return bar0 + 8u * (uint32_t)(2 * WS + NB + s); };
-    auto bar_tmem_full = [&](int b) { return bar0 + 8u * (uint32_t)(2 * WS + 2 * NB + b); };
-    auto bar_tmem_empty = [&](int b) { return bar0 + 8u * (uint32_t)(2 * WS + 2 * NB + SETS + b); };
+    auto bar_w_empty = [&](int s) { return bar0 + 8u * (uint32_t)(C::WS + s); };
+    auto bar_full = [&](int s) { return bar0 + 8u * (uint32_t)(2 * C::WS + s); };
+    auto bar_empty = [&](int s) { return bar0 + 8u * (uint32_t)(2 * C::WS + C::NB + s); };
+    auto bar_tmem_full = [&](int b) { return bar0 + 8u * (uint32_t)(2 * C::WS + 2 * C::NB + b); };
+    auto bar_tmem_empty = [&](int b) { return bar0 + 8u * (uint32_t)(2 * C::WS + 2 * C::NB + SETS + b); };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     pdl_trigger();
     if (threadIdx.x == 0) {
-        for (int s = 0; s < WS; s++) {
+        for (int s = 0; s < C::WS; s++) {
             mbar_init(bar_w_full(s), 1);
             mbar_init(bar_w_empty(s), GW);  // one elected arrival per warp of the decoding group
         }
-        for (int s = 0; s < NB; s++) {
+        for (int s = 0; s < C::NB; s++) {
             mbar_init(bar_full(s), GW + 1);  // the decode warps of a group + the TMA producer's expect_tx
             mbar_init(bar_empty(s), 1);     // tcgen05.commit
         }
@@ -231,8 +257,11 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
     tt.cnt = s_tables + (MAX_LOCAL_EXPERTS + 1);
     tt.tile_start = s_tables + 2 * (MAX_LOCAL_EXPERTS + 1);
 
+    auto next_unit = [](int bu, int need) {  // SB is a power of two where an item takes several units
+        return C::UNITS ? (bu + need) & (C::SB - 1) : (bu + 1 == C::SB ? 0 : bu + 1);
+    };
     const int total_tiles = tt.tile_start[E] * m_tiles;
-    const int n_steps = (k_stages + CS - 1) / CS;  // pipeline steps per work item; the last may hold fewer chunks
+    const int n_steps = (k_stages + C::CS - 1) / C::CS;  // pipeline steps per work item; the last may hold fewer chunks
 
     if (warp == 0) {
         // ------------------------- packed-weight producer ----------------------
@@ -243,7 +272,7 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
             int wstep = 0;
             (void)wstep;
             for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
-                const TileInfo ti = decode_tile(tile, m_tiles, tt, E);
+                const TileInfo ti = decode_tile<C>(tile, m_tiles, tt, E);
                 const uint8_t* wsrc = chunks + (size_t)ti.e * expert_stride +
                                       (size_t)ti.mt * k_stages * CHUNK_BYTES;
                 for (int st = 0; st < n_steps; st++) {
@@ -252,20 +281,20 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                         break;
                     TRACE(wstep, 0);
                     // the chunks of a weight tile are contiguous: one copy per step
-                    const uint32_t bytes = (uint32_t)(min(CS, k_stages - st * CS) * CHUNK_BYTES);
+                    const uint32_t bytes = (uint32_t)(min(C::CS, k_stages - st * C::CS) * CHUNK_BYTES);
                     mbar_expect_tx(bar_w_full(s), bytes);
-                    bulk_load(smem_u32(w_ring + s * W_SLOT_BYTES), wsrc + (size_t)st * W_SLOT_BYTES, bytes,
+                    bulk_load(smem_u32(w_ring + s * C::W_SLOT_BYTES), wsrc + (size_t)st * C::W_SLOT_BYTES, bytes,
                               bar_w_full(s));
                     TRACE(wstep, 1);
                     ++wstep;
-                    armed = min(armed + 1, WS);
-                    RING_ADVANCE(s, ph, WS);
+                    armed = min(armed + 1, C::WS);
+                    RING_ADVANCE(s, ph, C::WS);
                 }
             }
             if (!ok) {
                 for (int i = 0; i < armed; i++) {  // walk back over the copies in flight
                     if (--s < 0) {
-                        s = WS - 1;
+                        s = C::WS - 1;
                         ph ^= 1u;
                     }
                     drain_wait(bar_w_full(s), ph);
@@ -277,8 +306,8 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
         if (lane == 0) {
             // step i: barrier i % NB; its tiles take one or two units of the B ring (one copy:
             // a 3-d box of CS chunks).  Before a step is issued, step i - Q must be done, where Q
-            // is how many steps the ring is sure to hold: SBU while the last SBU steps all took
-            // one unit, SBU / 2 otherwise.  Steps finish in order, so the producer consumes the
+            // is how many steps the ring is sure to hold: SB while the last SB steps all took
+            // one unit, SB / 2 otherwise.  Steps finish in order, so the producer consumes the
             // empty barriers in step order.
             int i = 0, nb = 0, bu = 0, waited = 0, ones_run = 0;
             bool ok = true;
@@ -294,28 +323,37 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                     *abort_flag = 1;
             }
             for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
-                const TileInfo ti = decode_tile(tile, m_tiles, tt, E);
-                const int need = ti.n_mma >> 5;  // units per step: 1 or 2
+                const TileInfo ti = decode_tile<C>(tile, m_tiles, tt, E);
+                const int need = C::UNITS ? ti.n_mma >> 5 : 1;  // units per step: 1 or 2
+                const uint32_t tile_bytes = (32u << ti.box_idx) * 128u;
                 for (int st = 0; st < n_steps; st++, i++) {
-                    if (need == 2 && (bu & 1))
-                        bu = (bu + 1) & (SBU - 1);
+                    if (C::UNITS && need == 2 && (bu & 1))
+                        bu = (bu + 1) & (C::SB - 1);
                     ones_run = (need == 1) ? ones_run + 1 : 0;
-                    const int last = i - (ones_run > SBU ? SBU : SBU / 2);
+                    const int last = i - (!C::UNITS || ones_run > C::SB ? C::SB : C::SB / 2);
                     while (ok && waited <= last) {
-                        ok = mbar_wait(bar_empty(waited % NB), (uint32_t)(waited / NB) & 1u, status,
+                        ok = mbar_wait(bar_empty(waited % C::NB), (uint32_t)(waited / C::NB) & 1u, status,
                                        DS_TIMEOUT_EMPTY, abort_flag);
                         waited++;
                     }
                     if (!ok)
                         break;
                     TRACE(i, 2);
-                    // the whole box is delivered (chunks past the end of K arrive as zeros)
-                    mbar_expect_tx(bar_full(nb), (uint32_t)(CS * ti.n_mma) * 128u);
-                    tma_load_3d(smem_u32(b_ring + bu * B_UNIT_BYTES), &maps.box3[ti.box_idx], bar_full(nb), 0,
-                                ti.row0, st * CS);
+                    const uint32_t dst = smem_u32(b_ring + bu * C::B_SLOT_BYTES);
+                    if (C::UNITS) {
+                        // the whole box is delivered (chunks past the end of K arrive as zeros)
+                        mbar_expect_tx(bar_full(nb), (uint32_t)C::CS * tile_bytes);
+                        tma_load_3d(dst, &maps.box3[ti.box_idx], bar_full(nb), 0, ti.row0, st * C::CS);
+                    } else {
+                        const int nch = min(C::CS, k_stages - st * C::CS);
+                        mbar_expect_tx(bar_full(nb), (uint32_t)nch * tile_bytes);
+                        for (int j = 0; j < nch; j++)
+                            tma_load_2d(dst + (uint32_t)j * tile_bytes, &maps.box[ti.box_idx], bar_full(nb),
+                                        (st * C::CS + j) * KSTAGE, ti.row0);
+                    }
                     TRACE(i, 3);
-                    bu = (bu + need) & (SBU - 1);
-                    if (++nb == NB)
+                    bu = next_unit(bu, need);
+                    if (++nb == C::NB)
                         nb = 0;
                 }
             }
@@ -340,7 +378,7 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
         bool ok = true;
         int it = 0;
         for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++it) {
-            const TileInfo ti = decode_tile(tile, m_tiles, tt, E);
+            const TileInfo ti = decode_tile<C>(tile, m_tiles, tt, E);
             const int set = it % SETS, round = it / SETS;
             ok = mbar_wait(bar_tmem_empty(set), (uint32_t)(round & 1) ^ 1u, status,
                            DS_TIMEOUT_TMEM_EMPTY, abort_flag);
@@ -350,10 +388,10 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
             tc_fence_after();  // the epilogue's tcgen05.ld of this set came before
             if (lane == 0)
                 TRACE(it * n_steps, 12);
-            const uint32_t d_tmem = tmem_base + (uint32_t)(set * BN);
+            const uint32_t d_tmem = tmem_base + (uint32_t)(set * C::BN);
             const uint32_t idesc = make_idesc(ti.n_mma);
-            const int need = ti.n_mma >> 5;                    // B units per step
-            const uint32_t sub_step = (uint32_t)ti.n_mma * 8u;  // one chunk's tile in descriptor units of 16 bytes
+            const int need = C::UNITS ? ti.n_mma >> 5 : 1;     // B units per step
+            const uint32_t sub_step = (32u << ti.box_idx) * 8u;  // one chunk's tile in descriptor units of 16 bytes
             for (int st = 0; st < n_steps; st++) {
                 ok = mbar_wait_hot(bar_full(nb), ph, status, DS_TIMEOUT_FULL_A, abort_flag);
                 ok = __all_sync(0xffffffffu, ok);
@@ -362,16 +400,16 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                 if (lane == 0)
                     TRACE(it * n_steps + st, 4);
                 tc_fence_after();  // the decode warps' tcgen05.st of this step came before
-                const uint32_t a_tmem = tmem_base + (uint32_t)(TMEM_A0 + sa * A_SLOT_COLS);
-                if (need == 2 && (bu & 1))
-                    bu = (bu + 1) & (SBU - 1);
-                const uint64_t b_desc = make_sw128_desc(smem_u32(b_ring + bu * B_UNIT_BYTES));
+                const uint32_t a_tmem = tmem_base + (uint32_t)(C::TMEM_A0 + sa * C::A_SLOT_COLS);
+                if (C::UNITS && need == 2 && (bu & 1))
+                    bu = (bu + 1) & (C::SB - 1);
+                const uint64_t b_desc = make_sw128_desc(smem_u32(b_ring + bu * C::B_SLOT_BYTES));
                 const uint32_t b_lo = (uint32_t)b_desc, b_hi = (uint32_t)(b_desc >> 32);
-                const int nch = min(CS, k_stages - st * CS);
+                const int nch = min(C::CS, k_stages - st * C::CS);
                 if (elect_one_sync()) {
                     TRACE(it * n_steps + st, 13);
 #pragma unroll
-                    for (int j = 0; j < CS; j++) {
+                    for (int j = 0; j < C::CS; j++) {
                         if (j < nch) {
 #pragma unroll
                             for (int kk = 0; kk < KSTAGE / 16; kk++)
@@ -385,10 +423,10 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                 }
                 if (lane == 0)
                     TRACE(it * n_steps + st, 5);
-                RING_ADVANCE(nb, ph, NB);
-                if (++sa == SA)
+                RING_ADVANCE(nb, ph, C::NB);
+                if (++sa == C::SA)
                     sa = 0;
-                bu = (bu + need) & (SBU - 1);
+                bu = next_unit(bu, need);
             }
             if (ok && elect_one_sync())
                 umma_commit(bar_tmem_full(set));
@@ -404,25 +442,25 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
         const int g = u / (GW * 32);
         const int half = ((u >> 5) % GW) >> 2;  // 0: this warp takes chunks 0, 2, 4 of a step; 1: chunks 1, 3, 5
         const int r = (warp & 3) * 32 + lane;
-        const uint32_t a_lane = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)TMEM_A0;
+        const uint32_t a_lane = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)C::TMEM_A0;
         const int my_tiles = (int)blockIdx.x < total_tiles
                                  ? (total_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
         const int total_steps = my_tiles * n_steps;
         bool ok = true;
         for (int i = g; ok && i < total_steps; i += G) {
             // A slot i % SA is free when step i - SA is done: barrier (i - SA) % NB
-            const int sw = i % WS, sa = i % SA, nb = i % NB, eb = (i - SA + NB) % NB;
-            const uint32_t phw = (uint32_t)(i / WS) & 1u, phe = (uint32_t)((i - SA) / NB) & 1u;
+            const int sw = i % C::WS, sa = i % C::SA, nb = i % C::NB, eb = (i - C::SA + C::NB) % C::NB;
+            const uint32_t phw = (uint32_t)(i / C::WS) & 1u, phe = (uint32_t)((i - C::SA) / C::NB) & 1u;
             const int st = i % n_steps;  // step inside its work item
-            const int nch = min(CS, k_stages - st * CS);
+            const int nch = min(C::CS, k_stages - st * C::CS);
             ok = mbar_wait(bar_w_full(sw), phw, status, DS_TIMEOUT_FULL_W, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok)
                 break;
             if ((u & (GW * 32 - 1)) == 0)
                 TRACE(i, 6);
-            const unsigned char* wst = w_ring + sw * W_SLOT_BYTES;
-            const uint32_t a_slot = a_lane + (uint32_t)(sa * A_SLOT_COLS);
+            const unsigned char* wst = w_ring + sw * C::W_SLOT_BYTES;
+            const uint32_t a_slot = a_lane + (uint32_t)(sa * C::A_SLOT_COLS);
             bool slot_free = false;
             for (int j = half; j < nch; j += 2) {
                 const unsigned char* wc = wst + j * CHUNK_BYTES;
@@ -447,7 +485,7 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                     // ALU work overlaps the MMAs still reading it
                     if ((u & (GW * 32 - 1)) == 0)
                         TRACE(i, 7);
-                    if (i >= SA)
+                    if (i >= C::SA)
                         ok = mbar_wait(bar_empty(eb), phe, status, DS_TIMEOUT_EMPTY, abort_flag);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok)
@@ -468,12 +506,13 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                 __syncwarp();
                 if (lane == 0)
                     mbar_arrive(bar_w_empty(sw));
-                if (i >= SA)
+                if (i >= C::SA)
                     ok = mbar_wait(bar_empty(eb), phe, status, DS_TIMEOUT_EMPTY, abort_flag);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok)
                     break;
             }
+            tmem_st_wait();
             tc_fence_before();
             __syncwarp();
             if (lane == 0)
@@ -490,7 +529,7 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
         bool ok = true;
         int it = 0;
         for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++it) {
-            const TileInfo ti = decode_tile(tile, m_tiles, tt, E);
+            const TileInfo ti = decode_tile<C>(tile, m_tiles, tt, E);
             const int set = it % SETS, round = it / SETS;
             ok = mbar_wait(bar_tmem_full(set), (uint32_t)(round & 1), status, DS_TIMEOUT_TMEM_FULL,
                            abort_flag);
@@ -504,7 +543,7 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
             const float* be = bias + (size_t)ti.e * bias_stride;
             const float* rse = rscale + (size_t)ti.e * bias_stride;  // 2^shift of every weight row
             const int m = mt * TILE_M + row;
-            const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(set * BN);
+            const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(set * C::BN);
             if (MODE == 0) {
                 // Lanes 2p / 2p+1 hold the gate / up row of feature pair p.  After one
                 // exchange the even lane finishes columns c0..c0+15 of that feature and
@@ -520,7 +559,7 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                 const int st_idx = (odd ? 16 * 16 + 32 : 0) + (lane >> 1);
                 for (int c0 = 0; c0 < ti.n_mma; c0 += 32) {
                     float v[32];
-                    tmem_ld_sum<1, BN>(t_addr + (uint32_t)c0, v);
+                    tmem_ld_sum<1, C::BN>(t_addr + (uint32_t)c0, v);
 #pragma unroll
                     for (int c = 0; c < 16; c++) {
                         const float mine_lo = fmaf(v[c], rs, bm), mine_hi = fmaf(v[c + 16], rs, bm);
@@ -553,7 +592,7 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                 const bool m4_ok = m4 < out_rows_valid;                // the width is a multiple of 4
                 for (int c0 = 0; c0 < ti.n_mma; c0 += 32) {
                     float v[32];
-                    tmem_ld_sum<1, BN>(t_addr + (uint32_t)c0, v);
+                    tmem_ld_sum<1, C::BN>(t_addr + (uint32_t)c0, v);
 #pragma unroll
                     for (int half = 0; half < 2; half++) {
 #pragma unroll

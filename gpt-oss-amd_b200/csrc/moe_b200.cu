@@ -228,7 +228,13 @@ moe_b200_status check_layer(moe_b200_handle h, int layer) {
 }
 
 constexpr int TC5_BN = 256;                   // token rows per tile of the large-batch GEMM
-constexpr int SMALL_MAX_ROWS_PER_EXPERT = 64; // at most this many rows per expert on average: small-batch GEMM
+// Rows per expert on average up to which the small-batch GEMM takes 64-row and 128-row
+// items.  Measured (hidden 2880, us per layer, 64-row items / 128-row items / CTA pairs):
+// 32 experts, 384 tokens (48 rows) 187 / 200 / -, 512 (64 rows) 234 / 220 / -, 777 (97 rows)
+// - / 255 / 303; 128 experts, 3001 tokens (94 rows) - / 990 / 1104, 4096 (128 rows) -
+// / 1329 / 1206.
+constexpr int SMALL_MAX_ROWS_PER_EXPERT = 56;
+constexpr int WIDE_MAX_ROWS_PER_EXPERT = 112;
 
 // Token rows per routing block (16 x the router kernel's MT).  Measured (E = 128, route
 // stage in ms; block height, CTAs per cluster): 2048 tokens (16,1) 0.030, (32,1) 0.042,
@@ -452,30 +458,31 @@ moe_b200_status launch_pair(moe_b200_handle h, const LayerWeights& lw, const tc5
     return MOE_B200_OK;
 }
 
-// Small batches, decoded weights in tensor memory (gemm_tc5_ts.cuh).
+// Small batches, decoded weights in tensor memory (gemm_tc5_ts.cuh).  ATTR: bit of smem_attr_done.
+template <class C, int ATTR>
 moe_b200_status launch_ts(moe_b200_handle h, const LayerWeights& lw, const tc5::TensorMaps& maps_x,
                           const int* g_off, const int* g_cnt, const int* g_tile_start, float* yout,
                           const int* row_dst, const peer::GemmPeerIO& pio, cudaStream_t st) {
     const moe_b200_config& c = h->cfg;
     const int H = c.hidden_dim, I = c.intermediate_dim, EL = h->n_local;
     namespace ts = tc5::ts;
-    if (!(h->smem_attr_done & 32)) {
-        CU_TRY(h, cudaFuncSetAttribute(ts::expert_gemm_ts_kernel<0>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, ts::SMEM_BYTES));
-        CU_TRY(h, cudaFuncSetAttribute(ts::expert_gemm_ts_kernel<1>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, ts::SMEM_BYTES));
-        h->smem_attr_done |= 32;
+    if (!(h->smem_attr_done & ATTR)) {
+        CU_TRY(h, cudaFuncSetAttribute(ts::expert_gemm_ts_kernel<0, C>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+        CU_TRY(h, cudaFuncSetAttribute(ts::expert_gemm_ts_kernel<1, C>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+        h->smem_attr_done |= ATTR;
     }
     prof_mark(h, MOE_B200_STAGE_GEMM1, true, st);
     const bool pdl = c.ep_size == 1 && pdl_enabled();
-    CU_TRY(h, launch_kernel(pdl, ts::expert_gemm_ts_kernel<0>, dim3(h->n_sms), dim3(ts::N_THREADS),
-                            ts::SMEM_BYTES, st, maps_x, lw.w1, h->stride1, h->ks1, h->m_tiles1, lw.bias1,
+    CU_TRY(h, launch_kernel(pdl, ts::expert_gemm_ts_kernel<0, C>, dim3(h->n_sms), dim3(ts::N_THREADS),
+                            C::SMEM_BYTES, st, maps_x, lw.w1, h->stride1, h->ks1, h->m_tiles1, lw.bias1,
                             lw.rscale1, 2 * I, g_off, g_cnt, g_tile_start, EL, (void*)h->hbuf, I, I,
                             (const int*)nullptr, pio, c.swiglu_alpha, c.swiglu_limit, h->status));
     prof_mark(h, MOE_B200_STAGE_GEMM1, false, st);
     prof_mark(h, MOE_B200_STAGE_GEMM2, true, st);
-    CU_TRY(h, launch_kernel(pdl, ts::expert_gemm_ts_kernel<1>, dim3(h->n_sms), dim3(ts::N_THREADS),
-                            ts::SMEM_BYTES, st, h->maps_h, lw.w2, h->stride2, h->ks2, h->m_tiles2, lw.bias2,
+    CU_TRY(h, launch_kernel(pdl, ts::expert_gemm_ts_kernel<1, C>, dim3(h->n_sms), dim3(ts::N_THREADS),
+                            C::SMEM_BYTES, st, h->maps_h, lw.w2, h->stride2, h->ks2, h->m_tiles2, lw.bias2,
                             lw.rscale2, H, g_off, g_cnt, g_tile_start, EL, (void*)yout, H, H, row_dst, pio,
                             c.swiglu_alpha, c.swiglu_limit, h->status));
     prof_mark(h, MOE_B200_STAGE_GEMM2, false, st);
@@ -522,7 +529,9 @@ moe_b200_status launch_gemms(moe_b200_handle h, const LayerWeights& lw, const ui
     (void)I;
     (void)EL;
     if (bn == tc5::ts::BN)
-        return launch_ts(h, lw, maps_x, g_off, g_cnt, g_tile_start, yout, row_dst, pio, st);
+        return launch_ts<tc5::ts::Narrow, 32>(h, lw, maps_x, g_off, g_cnt, g_tile_start, yout, row_dst, pio, st);
+    if (bn == tc5::ts::BN_WIDE)
+        return launch_ts<tc5::ts::Wide, 128>(h, lw, maps_x, g_off, g_cnt, g_tile_start, yout, row_dst, pio, st);
     if (bn == TC5_BN)
         return launch_pair(h, lw, maps_x, g_off, g_cnt, g_tile_start, yout, row_dst, pio, st);
     return fail(h, MOE_B200_ERR_INVALID, "tile tables were built for another tile height");
@@ -546,7 +555,9 @@ int pick_bn(moe_b200_handle h, int rows) {
         return V0_BN;
 #endif
     const int per_expert = rows / (h->n_local > 0 ? h->n_local : 1);
-    return per_expert <= SMALL_MAX_ROWS_PER_EXPERT ? tc5::ts::BN : TC5_BN;
+    if (per_expert <= SMALL_MAX_ROWS_PER_EXPERT)
+        return tc5::ts::BN;
+    return per_expert <= WIDE_MAX_ROWS_PER_EXPERT ? tc5::ts::BN_WIDE : TC5_BN;
 }
 
 moe_b200_status check_shard(moe_b200_handle h, int first_expert, int n) {
@@ -961,7 +972,7 @@ moe_b200_status forward_impl(moe_b200_handle h, int layer, const void* t, int t_
     // Programmatic dependent launch pays for small batches (decode20b: 4.20 -> 4.05 ms per
     // step) and costs about 1 % on large ones (the next kernel's waiting blocks share the
     // SMs of a GEMM that is bound by instruction issue), so it follows the GEMM choice.
-    const bool pdl = c.ep_size == 1 && pdl_enabled() && bn_local == tc5::ts::BN;
+    const bool pdl = c.ep_size == 1 && pdl_enabled() && bn_local != TC5_BN;
     h->last_launches = 0;
     if (!h->prof_external)
         h->prof_call = (h->prof_next < h->prof_armed) ? h->prof_next++ : -1;
