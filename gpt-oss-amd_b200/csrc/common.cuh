@@ -151,10 +151,12 @@ __host__ __device__ __forceinline__ int ceil_div(int a, int b) { return (a + b -
 // does its own set-up (shared-memory init, barriers, tensor-memory allocation) and calls
 // pdl_wait() before it touches anything that kernel wrote -- the wait returns when the
 // whole previous grid has completed and its memory is visible.  pdl_trigger() lets the
-// NEXT kernel start its own set-up early; it orders nothing.  Both are no-ops in a
-// kernel launched the ordinary way.  Every kernel of the forward path calls both, in
-// this order, before its first global access that depends on an earlier kernel, and
-// writes nothing to global memory before the wait.
+// NEXT kernel start its own set-up early.  Both are no-ops in a kernel launched the
+// ordinary way.  Every kernel of the forward path calls both, and writes nothing to global
+// memory before the wait.
+// The kernels from the permute on trigger AFTER their wait.  So when the kernel behind one of
+// them starts, every kernel before that one has completed: the down GEMM may read the
+// plan, and the combine the routing, before their own wait.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -221,7 +221,6 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    pdl_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::WS; s++) {
             mbar_init(bar_w_full(s), 1);
@@ -240,9 +239,15 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
     }
     if (warp == MMA_WARP)
         tmem_alloc(smem_u32(tmem_holder), TMEM_COLS);
-    // everything above is this CTA's own set-up; what follows reads the plan, the token
-    // rows and the intermediate that earlier kernels of the call wrote
-    pdl_wait();
+    // Everything above is this CTA's own set-up.  The gate/up launch waits here: its plan and
+    // token rows come from the kernel before it.  Of what the down launch reads, only the
+    // intermediate does (the plan is complete when it starts, pdl_trigger in common.cuh), so
+    // there the activation producer and the epilogue wait, and weights stream and are decoded
+    // while the last gate/up CTAs still run.
+    if (MODE == 0) {
+        pdl_wait();
+        pdl_trigger();
+    }
     for (int i = threadIdx.x; i <= E; i += N_THREADS) {
         s_tables[i] = g_off[i];
         s_tables[(MAX_LOCAL_EXPERTS + 1) + i] = (i < E) ? g_cnt[i] : 0;
@@ -304,6 +309,10 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
     } else if (warp == 1) {
         // ------------------------- activation-tile producer --------------------
         if (lane == 0) {
+            if (MODE == 1) {
+                pdl_wait();
+                pdl_trigger();
+            }
             // step i: barrier i % NB; its tiles take one or two units of the B ring (one copy:
             // a 3-d box of CS chunks).  Before a step is issued, step i - Q must be done, where Q
             // is how many steps the ring is sure to hold: SB while the last SB steps all took
@@ -523,6 +532,8 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
     } else {
         // ------------------------------ epilogue ------------------------------
         // A lane holds one weight row (TMEM lane) for 32 token rows at a time.
+        if (MODE == 1)
+            pdl_wait();
         const int q = warp & 3;         // TMEM lane quarter this warp may read
         const int row = q * 32 + lane;  // row inside the weight tile
         unsigned char* stage = epi_stage + (warp - EPI_WARP0) * EPI_STAGE_BYTES;

@@ -106,14 +106,25 @@ permute_kernel(const void* __restrict__ x, int x_is_f32, int T, int H, int K, in
                const int* __restrict__ blk_hist, int nblk, int bn, int* __restrict__ cnt,
                int* __restrict__ off, int* __restrict__ tile_start) {
     __shared__ int s_base[256];
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
+    const int t0 = blockIdx.x * rb;  // rb <= RB tokens per block, the routing kernel's block size
+    const int n_assign = rb * K;
+    // this thread's assignments, fetched together with the histograms below
+    constexpr int AMAX = RB * 8 / 256;
+    int e_of[AMAX];
+#pragma unroll
+    for (int j = 0; j < AMAX; j++) {
+        const int a = threadIdx.x + j * 256;
+        e_of[j] = (a < n_assign && t0 + a / K < T) ? topk_i[(size_t)t0 * K + a] : -1;
+    }
     if (blk_hist) {
         __shared__ int s_tot[256];
         const int e = threadIdx.x;
         int before = 0;
         if (e < E) {
             int total = 0;
+#pragma unroll 8
             for (int b = 0; b < nblk; b++) {
                 const int v = blk_hist[(size_t)b * E + e];
                 before += (b < (int)blockIdx.x) ? v : 0;
@@ -162,19 +173,17 @@ permute_kernel(const void* __restrict__ x, int x_is_f32, int T, int H, int K, in
     }
     __shared__ int s_e[RB * 8];
     __shared__ int s_pos[RB * 8];
-    const int t0 = blockIdx.x * rb;  // rb <= RB tokens per block, the routing kernel's block size
-    const int n_assign = rb * K;
-    for (int a = threadIdx.x; a < n_assign; a += blockDim.x) {
-        const int t = t0 + a / K;
-        int e = -1;
-        if (t < T) {
-            e = topk_i[(size_t)t0 * K + a];
-            if (e < 0 || e >= E) {
+#pragma unroll
+    for (int j = 0; j < AMAX; j++) {
+        const int a = threadIdx.x + j * 256;
+        if (a < n_assign) {
+            int e = e_of[j];
+            if ((e < 0 || e >= E) && t0 + a / K < T) {
                 report_status(status, DS_BAD_EXPERT);
                 e = -1;
             }
+            s_e[a] = e;
         }
-        s_e[a] = e;
     }
     __syncthreads();
     // the gridDim.y blocks of a routing block split its TOKENS (all K assignments of a
@@ -250,37 +259,13 @@ combine_kernel(const float* __restrict__ y, int T, int H, int K, const int* __re
                const float* __restrict__ topk_w, const int* __restrict__ slot_of,
                float* __restrict__ out, int accumulate, const int* __restrict__ wait_flags, int G,
                int seq, int* __restrict__ status) {
-    pdl_trigger();
-    pdl_wait();
-    if (wait_flags) {
-        if ((int)threadIdx.x < G) {
-            const volatile int* f = wait_flags + threadIdx.x;
-            unsigned long long t_start = 0;
-            while ((int)(*f - seq) < 0) {
-                if (*reinterpret_cast<volatile int*>(status) != 0)
-                    break;
-                unsigned long long now;
-                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-                if (t_start == 0)
-                    t_start = now;
-                else if (now - t_start > 2000000000ull) {
-                    report_status(status, 0x301);  // peer::DS_TIMEOUT_PEER
-                    break;
-                }
-                __nanosleep(100);
-            }
-            __threadfence_system();
-        }
-        __syncthreads();
-    }
+    // the routing is two kernels old and more: complete before this kernel starts
     const int t = blockIdx.x;
-    if (t >= T)
-        return;
     int ex[8], sl[8];
     float wt[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-        if (k < K) {
+        if (k < K && t < T) {
             ex[k] = topk_i[(size_t)t * K + k];
             sl[k] = slot_of[(size_t)t * K + k];
             wt[k] = topk_w[(size_t)t * K + k];
@@ -302,6 +287,31 @@ combine_kernel(const float* __restrict__ y, int T, int H, int K, const int* __re
             }
         }
     }
+    pdl_wait();
+    pdl_trigger();
+    if (wait_flags) {
+        if ((int)threadIdx.x < G) {
+            const volatile int* f = wait_flags + threadIdx.x;
+            unsigned long long t_start = 0;
+            while ((int)(*f - seq) < 0) {
+                if (*reinterpret_cast<volatile int*>(status) != 0)
+                    break;
+                unsigned long long now;
+                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+                if (t_start == 0)
+                    t_start = now;
+                else if (now - t_start > 2000000000ull) {
+                    report_status(status, 0x301);  // peer::DS_TIMEOUT_PEER
+                    break;
+                }
+                __nanosleep(100);
+            }
+            __threadfence_system();
+        }
+        __syncthreads();
+    }
+    if (t >= T)
+        return;
     const int nvec = H / 4;
     float4* o = reinterpret_cast<float4*>(out + (size_t)t * H);
     for (int v = threadIdx.x; v < nvec; v += blockDim.x) {

@@ -159,6 +159,7 @@ __device__ __forceinline__ float rms_apply(float x, float w, float scale) {
 // between the sum of squares and the scaling (H <= 8192).
 constexpr int RCAST_THREADS = 256;
 constexpr int RCAST_MAX_VEC = 8;  // float4 per thread: H <= 8192
+constexpr int RCAST_EARLY_VEC = 4;
 
 __global__ void __launch_bounds__(RCAST_THREADS)
 rows_to_bf16_kernel(const float* __restrict__ x, int T, int H, const void* __restrict__ rms_w,
@@ -177,6 +178,24 @@ rows_to_bf16_kernel(const float* __restrict__ x, int T, int H, const void* __res
     for (int i = 0; i < RCAST_MAX_VEC; i++) {
         const int k = tid + i * RCAST_THREADS;
         v[i] = (k < nvec) ? row[k] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    auto weight = [&](int k) {
+        if (rms_w_is_f32)
+            return reinterpret_cast<const float4*>(rms_w)[k];
+        const uint2 wq = reinterpret_cast<const uint2*>(rms_w)[k];
+        return make_float4(__uint_as_float(wq.x << 16), __uint_as_float(wq.x & 0xFFFF0000u),
+                           __uint_as_float(wq.y << 16), __uint_as_float(wq.y & 0xFFFF0000u));
+    };
+    // the first weights are fetched with the row, not after the sum over it (rows of up to
+    // 4096 columns: all of them)
+    float4 wv[RCAST_EARLY_VEC];
+    if (rms_w) {
+#pragma unroll
+        for (int i = 0; i < RCAST_EARLY_VEC; i++) {
+            const int k = tid + i * RCAST_THREADS;
+            if (k < nvec)
+                wv[i] = weight(k);
+        }
     }
     float scale = 1.f;
     if (rms_w) {
@@ -213,17 +232,9 @@ rows_to_bf16_kernel(const float* __restrict__ x, int T, int H, const void* __res
         if (k < nvec) {
             float4 q = v[i];
             if (rms_w) {
-                float w0, w1, w2, w3;
-                if (rms_w_is_f32) {
-                    const float4 wq = reinterpret_cast<const float4*>(rms_w)[k];
-                    w0 = wq.x, w1 = wq.y, w2 = wq.z, w3 = wq.w;
-                } else {
-                    const uint2 wq = reinterpret_cast<const uint2*>(rms_w)[k];
-                    w0 = __uint_as_float(wq.x << 16), w1 = __uint_as_float(wq.x & 0xFFFF0000u);
-                    w2 = __uint_as_float(wq.y << 16), w3 = __uint_as_float(wq.y & 0xFFFF0000u);
-                }
-                q.x = rms_apply(q.x, w0, scale), q.y = rms_apply(q.y, w1, scale);
-                q.z = rms_apply(q.z, w2, scale), q.w = rms_apply(q.w, w3, scale);
+                const float4 w = i < RCAST_EARLY_VEC ? wv[i] : weight(k);
+                q.x = rms_apply(q.x, w.x, scale), q.y = rms_apply(q.y, w.y, scale);
+                q.z = rms_apply(q.z, w.z, scale), q.w = rms_apply(q.w, w.w, scale);
             }
             orow[k] = make_uint2(pack_bf16x2(q.x, q.y), pack_bf16x2(q.z, q.w));
         }
@@ -337,12 +348,13 @@ route_tc_kernel(const void* __restrict__ xv, int T, int H, const uint16_t* __res
             k -= n_chunks;
         return (crank + k * CS) * RMK;
     };
-    auto issue = [&](int c) {  // cp.async of the c-th chunk of this block into its stage
+    // cp.async of the c-th chunk of this block into its stage: its token rows, its router rows
+    auto issue = [&](int c, bool tokens, bool router) {
         uint16_t* st = tiles + (c % S) * STAGE_ELEMS;
         const int col = chunk_col(c);
 #pragma unroll
         for (int s = 0; s < SEGS; s++)
-            if (seg_src[s])
+            if (seg_src[s] && ((tid + s * RTHREADS) < RBT * 8 ? tokens : router))
                 cp_async_16(st + seg_dst[s], seg_src[s] + col);
     };
 
@@ -381,11 +393,19 @@ route_tc_kernel(const void* __restrict__ xv, int T, int H, const uint16_t* __res
         for (int i = 0; i < 4; i++)
             run[n][i] = 0.f;
 
-    pdl_wait();  // the rows may come from the kernel before this one
+    // The router matrix was uploaded before the call: its rows of the first chunks are on
+    // their way (from HBM, a layer's router is not in L2) while the kernel before this one
+    // still runs.  The token rows may come from that kernel.  A router row's copy belongs to
+    // the group of chunk 0, the oldest, so the waits below cover it.
+#pragma unroll
+    for (int c = 0; c < S - 1; c++)
+        if (c < n_chunks)
+            issue(c, false, true);
+    pdl_wait();
 #pragma unroll
     for (int c = 0; c < S - 1; c++) {
         if (c < n_chunks)
-            issue(c);
+            issue(c, true, false);
         cp_async_commit();
     }
     if (XF32) {
@@ -398,7 +418,7 @@ route_tc_kernel(const void* __restrict__ xv, int T, int H, const uint16_t* __res
         cp_async_wait<S - 2>();  // this thread's copies of chunk c have landed
         __syncthreads();         // everybody's have, and chunk c-1 is consumed
         if (c + S - 1 < n_chunks)
-            issue(c + S - 1);    // into the stage chunk c-1 just left
+            issue(c + S - 1, true, true);  // into the stage chunk c-1 just left
         cp_async_commit();
         if (XF32) {
             if (c + 1 < n_chunks)
