@@ -228,6 +228,9 @@ moe_b200_status check_layer(moe_b200_handle h, int layer) {
 }
 
 constexpr int TC5_BN = 256;                   // token rows per tile of the large-batch GEMM
+// Shared memory of front_small_kernel: hidden sizes up to 8192 with 32 experts, 5120 with 128,
+// 2560 with 256; beyond, the separate kernels run.
+constexpr int FRONT_MAX_SMEM = 220 * 1024;
 // Rows per expert on average up to which the small-batch GEMM takes 64-row and 128-row
 // items.  Measured (hidden 2880, us per layer, 64-row items / 128-row items / CTA pairs):
 // 32 experts, 384 tokens (48 rows) 187 / 200 / -, 512 (64 rows) 234 / 220 / -, 777 (97 rows)
@@ -381,6 +384,63 @@ cudaError_t launch_route(int dev, const RouteArgs& a, int rb, cudaStream_t st) {
     return cudaErrorInvalidValue;
 }
 
+// Up to 16 tokens: norm / cast, router, plan and permute in one launch (front_small_kernel).
+int g_front_attr[MAX_DEVICES];  // bit per NT instantiation
+
+template <int NT>
+cudaError_t launch_front_nt(moe_b200_handle h, const LayerWeights& lw, const void* t, int is_f32, const void* rms_w,
+                            int rms_w_is_f32, int T, int bn, float* score_out, bool pdl, cudaStream_t st) {
+    const moe_b200_config& c = h->cfg;
+    constexpr int bit = NT;
+    auto kernel = front_small_kernel<NT>;
+    if (!(g_front_attr[c.device] & bit)) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FRONT_MAX_SMEM);
+        if (e != cudaSuccess)
+            return e;
+        g_front_attr[c.device] |= bit;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(FRONT_CS);
+    cfg.blockDim = dim3(RTHREADS);
+    cfg.dynamicSmemBytes = front_smem_bytes<NT>(c.hidden_dim);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = FRONT_CS;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, t, is_f32, rms_w, rms_w_is_f32, T, c.hidden_dim,
+                              (const uint16_t*)lw.w_router, (const float*)lw.b_router, c.n_experts,
+                              c.experts_per_token, bn, score_out, h->topk_i, h->topk_w, h->slot_of, h->row_token,
+                              h->xs, h->cnt, h->off, h->tile_start, h->status);
+}
+
+// One routing block and one GPU.  At 17 tokens the copies of the permuted rows would already
+// want more than one cluster; expert parallelism places rows on other GPUs.
+bool front_fits(moe_b200_handle h, int T) {
+    const int nt = ceil_div(h->cfg.n_experts, 32), H = h->cfg.hidden_dim;
+    const size_t bytes = nt <= 1 ? front_smem_bytes<1>(H) : nt <= 2 ? front_smem_bytes<2>(H)
+                         : nt <= 4 ? front_smem_bytes<4>(H) : front_smem_bytes<8>(H);
+    return h->cfg.ep_size == 1 && h->cfg.device < MAX_DEVICES && T > 0 && T <= FRONT_MAX_T &&
+           H <= 4 * RCAST_THREADS * RCAST_MAX_VEC && bytes <= (size_t)FRONT_MAX_SMEM;
+}
+
+cudaError_t launch_front(moe_b200_handle h, const LayerWeights& lw, const void* t, int is_f32, const void* rms_w,
+                         int rms_w_is_f32, int T, int bn, float* score_out, bool pdl, cudaStream_t st) {
+    const int nt = ceil_div(h->cfg.n_experts, 32);
+    if (nt <= 1)
+        return launch_front_nt<1>(h, lw, t, is_f32, rms_w, rms_w_is_f32, T, bn, score_out, pdl, st);
+    if (nt <= 2)
+        return launch_front_nt<2>(h, lw, t, is_f32, rms_w, rms_w_is_f32, T, bn, score_out, pdl, st);
+    if (nt <= 4)
+        return launch_front_nt<4>(h, lw, t, is_f32, rms_w, rms_w_is_f32, T, bn, score_out, pdl, st);
+    return launch_front_nt<8>(h, lw, t, is_f32, rms_w, rms_w_is_f32, T, bn, score_out, pdl, st);
+}
+
 // Large batches on CTA pairs (gemm_tc5_pair.cuh): cluster launch, one cluster per SM pair.
 template <int MODE>
 moe_b200_status launch_pair_kernel(moe_b200_handle h, int grid, cudaStream_t st,
@@ -523,11 +583,11 @@ moe_b200_status launch_gemms(moe_b200_handle h, const LayerWeights& lw, const ui
         return MOE_B200_OK;
     }
 #endif
-    (void)xin;
     (void)rows_upper;
     (void)H;
     (void)I;
     (void)EL;
+    (void)xin;
     if (bn == tc5::ts::BN)
         return launch_ts<tc5::ts::Narrow, 32>(h, lw, maps_x, g_off, g_cnt, g_tile_start, yout, row_dst, pio, st);
     if (bn == tc5::ts::BN_WIDE)
@@ -977,7 +1037,14 @@ moe_b200_status forward_impl(moe_b200_handle h, int layer, const void* t, int t_
     if (!h->prof_external)
         h->prof_call = (h->prof_next < h->prof_armed) ? h->prof_next++ : -1;
 
-    if (T > 0) {
+    const bool front = front_fits(h, T);
+    if (front) {
+        prof_mark(h, MOE_B200_STAGE_ROUTE, true, s);
+        CU_TRY(h, launch_front(h, lw, t, (int)(t_dtype == MOE_B200_DTYPE_F32), rms_w,
+                               (int)(rms_w_dtype == MOE_B200_DTYPE_F32), T, bn_local, router_score_out, pdl, s));
+        prof_mark(h, MOE_B200_STAGE_ROUTE, false, s);
+        h->last_launches++;
+    } else if (T > 0) {
         prof_mark(h, MOE_B200_STAGE_ROUTE, true, s);
         if (t_dtype == MOE_B200_DTYPE_F32) {
             // fp32 rows (the engine's s->t, or with rms_w its residual stream) become the
@@ -1041,7 +1108,7 @@ moe_b200_status forward_impl(moe_b200_handle h, int layer, const void* t, int t_
         // small batches: the permute kernel plans by itself (one launch less on the
         // latency-bound path); otherwise a one-block plan kernel runs first
         const bool fused_plan = T > 0 && nblk <= PLAN_FUSED_MAX_BLOCKS;
-        if (fused_plan) {
+        if (fused_plan || front) {
             prof_mark(h, MOE_B200_STAGE_PLAN, true, s);  // an empty stage, not a stale one
             prof_mark(h, MOE_B200_STAGE_PLAN, false, s);
         } else {
@@ -1051,7 +1118,10 @@ moe_b200_status forward_impl(moe_b200_handle h, int layer, const void* t, int t_
             prof_mark(h, MOE_B200_STAGE_PLAN, false, s);
             h->last_launches++;
         }
-        if (T > 0) {
+        if (front) {
+            prof_mark(h, MOE_B200_STAGE_PERMUTE, true, s);
+            prof_mark(h, MOE_B200_STAGE_PERMUTE, false, s);
+        } else if (T > 0) {
             prof_mark(h, MOE_B200_STAGE_PERMUTE, true, s);
             CU_TRY(h, launch_kernel(pdl, permute_kernel, dim3(nblk, permute_split(h, nblk, rb * K)), dim3(256), 0,
                                     s, t, (int)(t_dtype == MOE_B200_DTYPE_F32), T, H, K, E, rb, h->topk_i,

@@ -74,11 +74,13 @@ constexpr size_t route_tc_smem_bytes() {
 // the K largest (ties to the lower index, src/hip/topk.hip:30-49), applies the
 // softmax over the selected logits (src/run.cpp:641, src/hip/softmax.hip:5-44),
 // stores indices and weights of token t and counts the experts in `hist`
-// (shared memory, integer adds: order-independent).
+// (shared memory, integer adds: order-independent); `list` (shared memory) takes the
+// indices too where a later step of the same kernel reads them.
 template <int NT>
 __device__ __forceinline__ void select_topk_softmax(float v[NT], int lane, int K, int t,
                                                     int* __restrict__ topk_i,
-                                                    float* __restrict__ topk_w, int* hist) {
+                                                    float* __restrict__ topk_w, int* hist,
+                                                    int* list = nullptr) {
     float sel_v[8];
     int sel_i[8];
 #pragma unroll
@@ -125,6 +127,8 @@ __device__ __forceinline__ void select_topk_softmax(float v[NT], int lane, int K
                 topk_i[(size_t)t * K + kk] = sel_i[kk];
                 topk_w[(size_t)t * K + kk] = ex[kk] / sum;
                 atomicAdd(&hist[sel_i[kk]], 1);
+                if (list)
+                    list[t * K + kk] = sel_i[kk];
             }
     }
 }
@@ -544,6 +548,270 @@ route_tc_kernel(const void* __restrict__ xv, int T, int H, const uint16_t* __res
     __syncthreads();
     for (int e = tid; e < E; e += RTHREADS)
         blk_hist[(size_t)tblk * E + e] = hist[e];
+}
+
+// ---------------------------------------------------------------------------
+// A batch of up to 16 tokens (one routing block): everything in front of the GEMMs in ONE
+// launch -- fp32 -> bf16 with the optional RMSNorm, router, top-K, softmax, plan, permute.
+// Such a call is a chain of latencies, and a launch boundary costs more than the work
+// behind it.  One cluster of FRONT_CS CTAs: CTA r keeps the token rows' and the router's chunks
+// r, r + FRONT_CS, ... in shared memory as a whole (no ring: 6 of 45 chunks at H = 2880), CTA 0
+// adds the partial logits in rank order and selects, as in route_tc_kernel with a K split (the
+// same operations in the same order: the same bits), plans, and every CTA stores its
+// columns of the permuted rows from shared memory, so the bf16 rows are never re-read.
+constexpr int FRONT_CS = 8;
+constexpr int FRONT_MAX_T = 16;
+
+template <int NT>
+__host__ __device__ constexpr size_t front_smem_bytes(int H) {
+    const int chunks = (H / RMK + FRONT_CS - 1) / FRONT_CS;
+    return (size_t)chunks * (FRONT_MAX_T + 32 * NT) * RMLD * 2 + (size_t)FRONT_MAX_T * 32 * NT * 4;
+}
+
+__device__ __forceinline__ int route_ld_remote_int(const int* p, uint32_t rank) {
+    int v;
+    const uint32_t la = (uint32_t)__cvta_generic_to_shared(p);
+    asm volatile(
+        "{\n\t.reg .b32 ra;\n\t"
+        "mapa.shared::cluster.u32 ra, %1, %2;\n\t"
+        "ld.shared::cluster.s32 %0, [ra];\n\t}"
+        : "=r"(v) : "r"(la), "r"(rank));
+    return v;
+}
+
+template <int NT>
+__global__ void __launch_bounds__(RTHREADS)
+front_small_kernel(const void* __restrict__ xv, int x_is_f32, const void* __restrict__ rms_w, int rms_w_is_f32,
+                   int T, int H, const uint16_t* __restrict__ w_router, const float* __restrict__ b_router, int E,
+                   int K, int bn, float* __restrict__ score_out, int* __restrict__ topk_i,
+                   float* __restrict__ topk_w, int* __restrict__ slot_of, int* __restrict__ row_token,
+                   uint16_t* __restrict__ xs_out, int* __restrict__ cnt, int* __restrict__ off,
+                   int* __restrict__ tile_start, int* __restrict__ status) {
+    constexpr int RBT = FRONT_MAX_T, EP = NT * 32, N_TILES = NT * 4, NG = 8, NTW = (N_TILES + NG - 1) / NG;
+    constexpr int ROWS = RBT + EP, STAGE_ELEMS = ROWS * RMLD;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int s_hist[256], s_base[256], s_e[RBT * 8], s_pos[RBT * 8];
+    __shared__ float s_scale[RBT];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+    const int crank = (int)route_cluster_rank();
+    const int n_all = H / RMK, n_chunks = (n_all - crank + FRONT_CS - 1) / FRONT_CS;
+    uint16_t* tiles = reinterpret_cast<uint16_t*>(smem_raw);
+    float* lg = reinterpret_cast<float*>(smem_raw + (size_t)((n_all + FRONT_CS - 1) / FRONT_CS) * STAGE_ELEMS * 2);
+
+    // router rows: uploaded before the call, so their copies start before the wait
+    for (int i = tid; i < n_chunks * EP * 8; i += RTHREADS) {
+        const int c = i / (EP * 8), e = (i >> 3) % EP, sg = i & 7;
+        uint16_t* dst = tiles + c * STAGE_ELEMS + (RBT + e) * RMLD + sg * 8;
+        if (e < E)
+            cp_async_16(dst, w_router + (size_t)e * H + (crank + c * FRONT_CS) * RMK + sg * 8);
+        else
+            *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
+    }
+    for (int i = tid; i < 256; i += RTHREADS)
+        s_hist[i] = 0;
+    pdl_wait();
+    pdl_trigger();
+
+    if (rms_w) {
+        // the CPU engine's norm (rms_apply): float products summed in double, one warp per row
+        for (int t = warp; t < T; t += RTHREADS / 32) {
+            const float4* row = reinterpret_cast<const float4*>(static_cast<const float*>(xv) + (size_t)t * H);
+            double ss = 0.0;
+#pragma unroll 8
+            for (int v = lane; v < H / 4; v += 32) {
+                const float4 q = row[v];
+                ss += (double)(q.x * q.x);
+                ss += (double)(q.y * q.y);
+                ss += (double)(q.z * q.z);
+                ss += (double)(q.w * q.w);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            if (lane == 0)
+                s_scale[t] = __fdiv_rn(1.0f, __fsqrt_rn((float)(ss / (double)H + (double)1e-5f)));
+        }
+        __syncthreads();
+    }
+    for (int i = tid; i < n_chunks * RBT * 8; i += RTHREADS) {
+        const int c = i / (RBT * 8), t = (i >> 3) % RBT, sg = i & 7;
+        const int col = (crank + c * FRONT_CS) * RMK + sg * 8;
+        uint16_t* dst = tiles + c * STAGE_ELEMS + t * RMLD + sg * 8;
+        if (t < T && !x_is_f32) {
+            cp_async_16(dst, static_cast<const uint16_t*>(xv) + (size_t)t * H + col);
+            continue;
+        }
+        uint4 r = make_uint4(0, 0, 0, 0);
+        if (t < T) {
+            const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(xv) + (size_t)t * H + col);
+            float v[8];
+            *reinterpret_cast<float4*>(v) = p[0];
+            *reinterpret_cast<float4*>(v + 4) = p[1];
+            if (rms_w) {
+                const float scale = s_scale[t];
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const float w = rms_w_is_f32
+                                        ? static_cast<const float*>(rms_w)[col + j]
+                                        : bf16_bits_to_float(static_cast<const uint16_t*>(rms_w)[col + j]);
+                    v[j] = rms_apply(v[j], w, scale);
+                }
+            }
+            r = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]),
+                           pack_bf16x2(v[6], v[7]));
+        }
+        *reinterpret_cast<uint4*>(dst) = r;
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+
+    float run[NTW][4];
+#pragma unroll
+    for (int n = 0; n < NTW; n++)
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            run[n][i] = 0.f;
+    for (int c = 0; c < n_chunks; c++) {
+        const uint16_t* xs = tiles + c * STAGE_ELEMS;
+        const uint16_t* ws = xs + RBT * RMLD;
+        float acc[NTW][4];
+#pragma unroll
+        for (int n = 0; n < NTW; n++)
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                acc[n][i] = 0.f;
+#pragma unroll
+        for (int kk = 0; kk < RMK / 16; kk++) {
+            uint32_t af[4];
+            const uint16_t* pa = xs + g * RMLD + kk * 16 + 2 * t4;
+            af[0] = *reinterpret_cast<const uint32_t*>(pa);
+            af[1] = *reinterpret_cast<const uint32_t*>(pa + 8 * RMLD);
+            af[2] = *reinterpret_cast<const uint32_t*>(pa + 8);
+            af[3] = *reinterpret_cast<const uint32_t*>(pa + 8 * RMLD + 8);
+#pragma unroll
+            for (int n = 0; n < NTW; n++) {
+                const int nt = warp * NTW + n;
+                if (nt < N_TILES) {
+                    const uint16_t* pb = ws + (nt * 8 + g) * RMLD + kk * 16 + 2 * t4;
+                    uint32_t bf[2];
+                    bf[0] = *reinterpret_cast<const uint32_t*>(pb);
+                    bf[1] = *reinterpret_cast<const uint32_t*>(pb + 8);
+                    route_mma_16816(acc[n], af, bf);
+                }
+            }
+        }
+#pragma unroll
+        for (int n = 0; n < NTW; n++)
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                run[n][i] += acc[n][i];
+    }
+#pragma unroll
+    for (int n = 0; n < NTW; n++) {
+        const int nt = warp * NTW + n;
+        if (nt < N_TILES) {
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                lg[(g + 8 * (i >> 1)) * EP + nt * 8 + 2 * t4 + (i & 1)] = run[n][i];
+        }
+    }
+    route_cluster_sync();  // every CTA's partial sums are in its shared memory
+    if (crank == 0) {
+        float4* lg4 = reinterpret_cast<float4*>(lg);
+        for (int i = tid; i < T * EP / 4; i += RTHREADS) {
+            float4 part[FRONT_CS];
+            part[0] = lg4[i];
+#pragma unroll
+            for (int r = 1; r < FRONT_CS; r++)
+                part[r] = route_ld_remote(lg4 + i, (uint32_t)r);
+            float4 v = part[0];
+#pragma unroll
+            for (int r = 1; r < FRONT_CS; r++) {
+                v.x += part[r].x;
+                v.y += part[r].y;
+                v.z += part[r].z;
+                v.w += part[r].w;
+            }
+            const int e = (4 * i) % EP;
+            v.x = (e + 0 < E) ? v.x + b_router[e + 0] : -INFINITY;
+            v.y = (e + 1 < E) ? v.y + b_router[e + 1] : -INFINITY;
+            v.z = (e + 2 < E) ? v.z + b_router[e + 2] : -INFINITY;
+            v.w = (e + 3 < E) ? v.w + b_router[e + 3] : -INFINITY;
+            lg4[i] = v;
+        }
+        __syncthreads();
+        if (score_out)
+            for (int i = tid; i < T * E; i += RTHREADS)
+                score_out[i] = lg[(i / E) * EP + i % E];
+        for (int t = warp; t < T; t += RTHREADS / 32) {
+            float v[NT];
+#pragma unroll
+            for (int j = 0; j < NT; j++)
+                v[j] = lg[t * EP + lane + 32 * j];
+            select_topk_softmax<NT>(v, lane, K, t, topk_i, topk_w, s_hist, s_e);
+        }
+        __syncthreads();
+        if (warp == 0) {
+            // exclusive prefix over the experts and over their tile counts
+            int carry_o = 0, carry_t = 0;
+            for (int e0 = 0; e0 < E; e0 += 32) {
+                const int i = e0 + lane, c = i < E ? s_hist[i] : 0, ntl = (c + bn - 1) / bn;
+                int so = c, stl = ntl;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int uo = __shfl_up_sync(0xffffffffu, so, d), ut = __shfl_up_sync(0xffffffffu, stl, d);
+                    if (lane >= d) {
+                        so += uo;
+                        stl += ut;
+                    }
+                }
+                if (i < E) {
+                    s_base[i] = carry_o + so - c;
+                    cnt[i] = c;
+                    off[i] = carry_o + so - c;
+                    tile_start[i] = carry_t + stl - ntl;
+                }
+                carry_o += __shfl_sync(0xffffffffu, so, 31);
+                carry_t += __shfl_sync(0xffffffffu, stl, 31);
+            }
+            if (lane == 0) {
+                off[E] = carry_o;
+                tile_start[E] = carry_t;
+            }
+        }
+        __syncthreads();
+        for (int a = tid; a < T * K; a += RTHREADS) {  // stable: token order inside an expert
+            const int e = s_e[a];
+            int pos = -1;
+            if (e < 0 || e >= E) {
+                report_status(status, DS_BAD_EXPERT);
+            } else {
+                pos = s_base[e];
+                for (int j = 0; j < a; j++)
+                    pos += s_e[j] == e;
+                slot_of[a] = pos;
+                row_token[pos] = a / K;
+            }
+            s_pos[a] = pos;
+        }
+    }
+    route_cluster_sync();  // the positions are in CTA 0's shared memory
+    if (crank != 0) {
+        for (int a = tid; a < T * K; a += RTHREADS)
+            s_pos[a] = route_ld_remote_int(s_pos + a, 0);
+    }
+    route_cluster_sync();  // they have been read: CTA 0 may leave
+    for (int i = tid; i < n_chunks * T * 8; i += RTHREADS) {
+        const int sg = i & 7, c = (i >> 3) % n_chunks, t = (i >> 3) / n_chunks;
+        const uint4 v = *reinterpret_cast<const uint4*>(tiles + c * STAGE_ELEMS + t * RMLD + sg * 8);
+        const int col = (crank + c * FRONT_CS) * RMK + sg * 8;
+        for (int k = 0; k < K; k++) {
+            const int pos = s_pos[t * K + k];
+            if (pos >= 0)
+                *reinterpret_cast<uint4*>(xs_out + (size_t)pos * H + col) = v;
+        }
+    }
 }
 
 }  // namespace moe
