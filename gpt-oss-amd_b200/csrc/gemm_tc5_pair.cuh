@@ -118,7 +118,6 @@ struct TileInfo {
     int row0;     // first token row of the item
     int valid_n;  // token rows of the item (1..256)
     int n_mma;    // rows the MMA computes (a multiple of 32)
-    int box_idx;  // TMA box for this CTA's half: 32 << box_idx rows
 };
 
 struct TileTables {
@@ -158,8 +157,6 @@ __device__ __forceinline__ TileInfo decode_tile(int tile, int m_pairs, const Til
     ti.row0 = tt.off[lo] + n0;
     ti.valid_n = min(rows, cnt - n0);
     ti.n_mma = max(32, (ti.valid_n + 31) & ~31);
-    const int nh = ti.n_mma >> 1;
-    ti.box_idx = nh <= 32 ? 0 : nh <= 64 ? 1 : 2;
     return ti;
 }
 
@@ -314,8 +311,8 @@ expert_gemm_pair_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* 
                         RING_ADVANCE(eb, phe, NB);
                     }
                     TRACE(i, 2);
-                    mbar_expect_tx(bar_full(nb), (uint32_t)(32 << ti.box_idx) * 128u);
-                    tma_load_2d(smem_u32(b_ring + sb * B_SLOT_BYTES), &maps.box[ti.box_idx],
+                    mbar_expect_tx(bar_full(nb), (uint32_t)(ti.n_mma >> 1) * 128u);
+                    tma_load_2d(smem_u32(b_ring + sb * B_SLOT_BYTES), &maps.box[(ti.n_mma >> 5) - 1],
                                 bar_full(nb), ks * KSTAGE, half_row0);
                     TRACE(i, 3);
                     if (++sb == SB)

@@ -143,8 +143,7 @@ struct TileInfo {
     int mt;       // 128-row weight tile
     int row0;     // first token row of the item
     int valid_n;  // token rows of the item (1..64)
-    int n_mma;    // rows the MMA computes (a multiple of 32)
-    int box_idx;  // TMA box: 32 << box_idx rows
+    int n_mma;    // rows the MMA computes and the TMA box holds (a multiple of 16)
 };
 
 struct TileTables {
@@ -181,8 +180,7 @@ __device__ __forceinline__ TileInfo decode_tile(int tile, int m_tiles, const Til
     const int n0 = (r - ti.mt * ntl) * rows;
     ti.row0 = tt.off[lo] + n0;
     ti.valid_n = min(rows, cnt - n0);
-    ti.n_mma = max(32, (ti.valid_n + 31) & ~31);
-    ti.box_idx = ti.n_mma <= 32 ? 0 : ti.n_mma <= 64 ? 1 : 2;
+    ti.n_mma = (ti.valid_n + 15) & ~15;
     return ti;
 }
 
@@ -333,8 +331,8 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
             }
             for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
                 const TileInfo ti = decode_tile<C>(tile, m_tiles, tt, E);
-                const int need = C::UNITS ? ti.n_mma >> 5 : 1;  // units per step: 1 or 2
-                const uint32_t tile_bytes = (32u << ti.box_idx) * 128u;
+                const int need = C::UNITS ? (ti.n_mma + 31) >> 5 : 1;  // units per step: 1 or 2
+                const uint32_t tile_bytes = (uint32_t)ti.n_mma * 128u;
                 for (int st = 0; st < n_steps; st++, i++) {
                     if (C::UNITS && need == 2 && (bu & 1))
                         bu = (bu + 1) & (C::SB - 1);
@@ -352,12 +350,12 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                     if (C::UNITS) {
                         // the whole box is delivered (chunks past the end of K arrive as zeros)
                         mbar_expect_tx(bar_full(nb), (uint32_t)C::CS * tile_bytes);
-                        tma_load_3d(dst, &maps.box3[ti.box_idx], bar_full(nb), 0, ti.row0, st * C::CS);
+                        tma_load_3d(dst, &maps.box3[(ti.n_mma >> 4) - 1], bar_full(nb), 0, ti.row0, st * C::CS);
                     } else {
                         const int nch = min(C::CS, k_stages - st * C::CS);
                         mbar_expect_tx(bar_full(nb), (uint32_t)nch * tile_bytes);
                         for (int j = 0; j < nch; j++)
-                            tma_load_2d(dst + (uint32_t)j * tile_bytes, &maps.box[ti.box_idx], bar_full(nb),
+                            tma_load_2d(dst + (uint32_t)j * tile_bytes, &maps.box[(ti.n_mma >> 4) - 1], bar_full(nb),
                                         (st * C::CS + j) * KSTAGE, ti.row0);
                     }
                     TRACE(i, 3);
@@ -399,8 +397,8 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                 TRACE(it * n_steps, 12);
             const uint32_t d_tmem = tmem_base + (uint32_t)(set * C::BN);
             const uint32_t idesc = make_idesc(ti.n_mma);
-            const int need = C::UNITS ? ti.n_mma >> 5 : 1;     // B units per step
-            const uint32_t sub_step = (32u << ti.box_idx) * 8u;  // one chunk's tile in descriptor units of 16 bytes
+            const int need = C::UNITS ? (ti.n_mma + 31) >> 5 : 1;  // B units per step
+            const uint32_t sub_step = (uint32_t)ti.n_mma * 8u;  // one chunk's tile in descriptor units of 16 bytes
             for (int st = 0; st < n_steps; st++) {
                 ok = mbar_wait_hot(bar_full(nb), ph, status, DS_TIMEOUT_FULL_A, abort_flag);
                 ok = __all_sync(0xffffffffu, ok);

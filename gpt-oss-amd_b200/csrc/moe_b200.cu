@@ -191,10 +191,10 @@ moe_b200_status make_maps(moe_b200_handle h, tc5::TensorMaps* maps, void* base, 
     if (!fn || qres != cudaDriverEntryPointSuccess)
         return fail(h, MOE_B200_ERR_CUDA, "cuTensorMapEncodeTiled not available in this driver");
     EncodeTiledFn encode = reinterpret_cast<EncodeTiledFn>(fn);
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < 8; i++) {
         cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
         cuuint64_t strides[1] = {(cuuint64_t)cols * 2};
-        cuuint32_t box[2] = {(cuuint32_t)KSTAGE, (cuuint32_t)(32 << i)};
+        cuuint32_t box[2] = {(cuuint32_t)KSTAGE, (cuuint32_t)(16 * (i + 1))};
         cuuint32_t estr[2] = {1, 1};
         CUresult r = encode(&maps->box[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides,
                             box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -203,11 +203,11 @@ moe_b200_status make_maps(moe_b200_handle h, tc5::TensorMaps* maps, void* base, 
             return fail(h, MOE_B200_ERR_CUDA,
                         "cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
     }
-    for (int i = 0; i < 2; i++) {
+    for (int i = 0; i < 4; i++) {
         // [chunk][row][64 columns]: the chunk axis has the smallest stride (128 bytes)
         cuuint64_t dims[3] = {(cuuint64_t)KSTAGE, (cuuint64_t)rows, (cuuint64_t)(cols / KSTAGE)};
         cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)KSTAGE * 2};
-        cuuint32_t box[3] = {(cuuint32_t)KSTAGE, (cuuint32_t)(32 << i), (cuuint32_t)tc5::STEP_CHUNKS};
+        cuuint32_t box[3] = {(cuuint32_t)KSTAGE, (cuuint32_t)(16 * (i + 1)), (cuuint32_t)tc5::STEP_CHUNKS};
         cuuint32_t estr[3] = {1, 1, 1};
         CUresult r = encode(&maps->box3[i], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, dims, strides,
                             box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,

@@ -15,10 +15,15 @@ constexpr uint32_t WAIT_SUSPEND_NS = 20000;                 // one suspended tes
 constexpr int STEP_CHUNKS = 6;  // 64-column chunks per pipeline step of the small-batch GEMM
 
 struct TensorMaps {
-    CUtensorMap box[4];   // token-row boxes of 32, 64, 128 (and 256, unused) rows x 64 columns
-    // the same rows seen as [chunk of 64 columns][row][64 columns]: boxes of 32 and 64 rows x
-    // STEP_CHUNKS chunks, so that one copy brings the activation tiles of a whole step
-    CUtensorMap box3[2];
+    // Token-row boxes of 16 (i + 1) rows x 64 columns.  A tile is loaded with the rows that
+    // its MMA computes and no more: at the decode rate the activations of a step weigh as much as
+    // its packed weights on the way from L2.  Against boxes of 32, 64 and 128 rows (us per
+    // layer, hidden 2880): 200 tokens x 128 experts 521 -> 479, 128 tokens x 32 147 -> 135,
+    // 3001 x 128 991 -> 945, 16384 x 128 3468 -> 3356.
+    CUtensorMap box[8];
+    // the same rows seen as [chunk of 64 columns][row][64 columns]: boxes of 16 (i + 1)
+    // rows x STEP_CHUNKS chunks, so that one copy brings the activation tiles of a whole step
+    CUtensorMap box3[4];
 };
 
 // ---------------------------------------------------------------------------
