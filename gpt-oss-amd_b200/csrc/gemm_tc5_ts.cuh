@@ -540,6 +540,13 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
         for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++it) {
             const TileInfo ti = decode_tile<C>(tile, m_tiles, tt, E);
             const int set = it % SETS, round = it / SETS;
+            // Bias and 2^shift of this lane's weight row, cold in HBM: fetched while the MMAs of
+            // the item run, so that the last item of a launch does not wait for them.
+            const int mt = ti.mt;
+            const int m = mt * TILE_M + row;
+            const bool m_ok = MODE == 0 || m < out_rows_valid;  // 2I is a multiple of TILE_M: always in range
+            const float bm = m_ok ? __ldg(bias + (size_t)ti.e * bias_stride + m) : 0.f;
+            const float rs = m_ok ? __ldg(rscale + (size_t)ti.e * bias_stride + m) : 1.f;
             ok = mbar_wait(bar_tmem_full(set), (uint32_t)(round & 1), status, DS_TIMEOUT_TMEM_FULL,
                            abort_flag);
             ok = __all_sync(0xffffffffu, ok);
@@ -548,10 +555,6 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
             if (warp == EPI_WARP0 && lane == 0)
                 TRACE(it * n_steps, 10);
             tc_fence_after();
-            const int mt = ti.mt;
-            const float* be = bias + (size_t)ti.e * bias_stride;
-            const float* rse = rscale + (size_t)ti.e * bias_stride;  // 2^shift of every weight row
-            const int m = mt * TILE_M + row;
             const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(set * C::BN);
             if (MODE == 0) {
                 // Lanes 2p / 2p+1 hold the gate / up row of feature pair p.  After one
@@ -561,7 +564,6 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                 // store writes 16 bytes per lane.
                 uint16_t* h = static_cast<uint16_t*>(outp);
                 uint16_t* stage16 = reinterpret_cast<uint16_t*>(stage);
-                const float bm = be[m], rs = rse[m];  // 2I is a multiple of TILE_M: always in range
                 const int jf0 = (mt * TILE_M + q * 32) >> 1;  // first of this warp's 16 features
                 const bool odd = (lane & 1) != 0;
                 // token rows 16..31 sit 64 bytes further: no bank conflict between the halves
@@ -595,8 +597,6 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                 // bytes and a warp instruction four whole 128-byte row segments.
                 float* y = static_cast<float*>(outp);
                 float* stage32 = reinterpret_cast<float*>(stage);
-                const float bm = (m < out_rows_valid) ? be[m] : 0.f;
-                const float rs = (m < out_rows_valid) ? rse[m] : 1.f;
                 const int m4 = mt * TILE_M + q * 32 + (lane & 7) * 4;  // columns this lane stores
                 const bool m4_ok = m4 < out_rows_valid;                // the width is a multiple of 4
                 for (int c0 = 0; c0 < ti.n_mma; c0 += 32) {

@@ -1161,7 +1161,8 @@ moe_b200_status forward_impl(moe_b200_handle h, int layer, const void* t, int t_
         // peer mode launches it for T == 0 as well: the wait inside is what orders this
         // rank's next call behind the peers' reads of this one
         prof_mark(h, MOE_B200_STAGE_COMBINE, true, s);
-        CU_TRY(h, launch_kernel(pdl, combine_kernel, dim3(T > 0 ? T : 1), dim3(256), 0, s, y_for_combine, T, H,
+        const int combine_split = T <= 2 * h->n_sms && !peer_mode ? ceil_div(H / 4, 256) : 1;
+        CU_TRY(h, launch_kernel(pdl, combine_kernel, dim3(T > 0 ? T : 1, combine_split), dim3(256), 0, s, y_for_combine, T, H,
                                 K, h->topk_i, h->topk_w, h->slot_of, out, accumulate, combine_wait, c.ep_size,
                                 seq, h->status));
         prof_mark(h, MOE_B200_STAGE_COMBINE, false, s);

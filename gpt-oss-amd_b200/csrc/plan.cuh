@@ -248,7 +248,8 @@ permute_kernel(const void* __restrict__ x, int x_is_f32, int T, int H, int K, in
 }
 
 // out[t,:] (+)= sum over the token's K assignments, ascending expert index, of
-// topk_w * y[slot,:].  One block per token.
+// topk_w * y[slot,:].  gridDim.y blocks per token: one, or for a few tokens as many as
+// leave one vector to a thread, since the kernel is then a chain of load latencies.
 // Expert-parallel peer mode: `wait_flags` points at this rank's G "results
 // delivered" flags; the block first waits (bounded) until every rank has stored
 // its result rows into y.  The grid then has at least one block even for T == 0:
@@ -314,7 +315,7 @@ combine_kernel(const float* __restrict__ y, int T, int H, int K, const int* __re
         return;
     const int nvec = H / 4;
     float4* o = reinterpret_cast<float4*>(out + (size_t)t * H);
-    for (int v = threadIdx.x; v < nvec; v += blockDim.x) {
+    for (int v = blockIdx.y * blockDim.x + threadIdx.x; v < nvec; v += gridDim.y * blockDim.x) {
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int k = 0; k < 8; k++) {
