@@ -156,9 +156,28 @@ __host__ __device__ __forceinline__ int ceil_div(int a, int b) { return (a + b -
 // memory before the wait.
 // The kernels from the permute on trigger AFTER their wait.  So when the kernel behind one of
 // them starts, every kernel before that one has completed: the down GEMM may read the
-// plan, and the combine the routing, before their own wait.
+// plan, and the combine the routing, before their own wait -- through ld_l2() only.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// A load before this kernel's own pdl_wait(), of what a kernel two or more back stored.
+// Guaranteed: that kernel has completed (above), and the kernel between the two waited for it,
+// so its stores are performed and visible to a grid on any SM, that is, they are in L2.  Not
+// guaranteed is that a plain load of THIS kernel sees them before its own wait: the same
+// workspace is written in every call, and a plain or read-only load may be answered from an L1
+// line of an earlier one.  A relaxed load of gpu scope is performed at L2, where all SMs agree on
+// the value; it costs what a load that misses L1 costs.  (Assumed, since PTX names no ordering
+// for it: a trigger is not seen by the dependent launch before it is executed.)
+__device__ __forceinline__ int ld_l2(const int* p) {
+    int v;
+    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ float ld_l2(const float* p) {
+    float v;
+    asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
 
 // Clamped SwiGLU (src/run.cpp:673-689, src/hip/moe.hip:186-191): the gate has no
 // lower clamp.

@@ -241,15 +241,15 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
     // token rows come from the kernel before it.  Of what the down launch reads, only the
     // intermediate does (the plan is complete when it starts, pdl_trigger in common.cuh), so
     // there the activation producer and the epilogue wait, and weights stream and are decoded
-    // while the last gate/up CTAs still run.
+    // while the last gate/up CTAs still run; the plan is read past L1 (ld_l2).
     if (MODE == 0) {
         pdl_wait();
         pdl_trigger();
     }
     for (int i = threadIdx.x; i <= E; i += N_THREADS) {
-        s_tables[i] = g_off[i];
-        s_tables[(MAX_LOCAL_EXPERTS + 1) + i] = (i < E) ? g_cnt[i] : 0;
-        s_tables[2 * (MAX_LOCAL_EXPERTS + 1) + i] = g_tile_start[i];
+        s_tables[i] = ld_l2(g_off + i);
+        s_tables[(MAX_LOCAL_EXPERTS + 1) + i] = (i < E) ? ld_l2(g_cnt + i) : 0;
+        s_tables[2 * (MAX_LOCAL_EXPERTS + 1) + i] = ld_l2(g_tile_start + i);
     }
     tc_fence_before();
     __syncthreads();

@@ -260,16 +260,17 @@ combine_kernel(const float* __restrict__ y, int T, int H, int K, const int* __re
                const float* __restrict__ topk_w, const int* __restrict__ slot_of,
                float* __restrict__ out, int accumulate, const int* __restrict__ wait_flags, int G,
                int seq, int* __restrict__ status) {
-    // the routing is two kernels old and more: complete before this kernel starts
+    // the routing is two kernels old and more: complete before this kernel starts, and read past
+    // L1 because this kernel has not waited yet (ld_l2)
     const int t = blockIdx.x;
     int ex[8], sl[8];
     float wt[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) {
         if (k < K && t < T) {
-            ex[k] = topk_i[(size_t)t * K + k];
-            sl[k] = slot_of[(size_t)t * K + k];
-            wt[k] = topk_w[(size_t)t * K + k];
+            ex[k] = ld_l2(topk_i + (size_t)t * K + k);
+            sl[k] = ld_l2(slot_of + (size_t)t * K + k);
+            wt[k] = ld_l2(topk_w + (size_t)t * K + k);
         } else {
             ex[k] = 0x7fffffff;
             sl[k] = 0;
