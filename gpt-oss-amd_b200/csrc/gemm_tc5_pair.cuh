@@ -200,7 +200,6 @@ expert_gemm_pair_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* 
     const uint32_t rank = cluster_ctarank();  // 0 = leader: issues the MMAs
     const bool leader = rank == 0;
 
-    pdl_trigger();
     if (threadIdx.x == 0) {
         for (int s = 0; s < WS; s++) {
             mbar_init(bar_w_full(s), 1);
@@ -223,6 +222,7 @@ expert_gemm_pair_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* 
     // everything above is this CTA's own set-up; what follows reads the plan, the token
     // rows and the intermediate that earlier kernels of the call wrote
     pdl_wait();
+    pdl_trigger();
     for (int i = threadIdx.x; i <= E; i += N_THREADS) {
         s_tables[i] = g_off[i];
         s_tables[(MAX_LOCAL_EXPERTS + 1) + i] = (i < E) ? g_cnt[i] : 0;

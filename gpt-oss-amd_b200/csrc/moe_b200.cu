@@ -1032,6 +1032,8 @@ moe_b200_status forward_impl(moe_b200_handle h, int layer, const void* t, int t_
     // Programmatic dependent launch pays for small batches (decode20b: 4.20 -> 4.05 ms per
     // step) and costs about 1 % on large ones (the next kernel's waiting blocks share the
     // SMs of a GEMM that is bound by instruction issue), so it follows the GEMM choice.
+    // The down GEMM and the combine read the plan and the routing before their wait, which
+    // rests on every kernel behind the router triggering after its own (common.cuh).
     const bool pdl = c.ep_size == 1 && pdl_enabled() && bn_local != TC5_BN;
     h->last_launches = 0;
     if (!h->prof_external)

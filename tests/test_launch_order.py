@@ -17,7 +17,7 @@ def kernel_body(file, name):
     with open(os.path.join(CSRC, file)) as f:
         src = f.read()
     src = re.sub(r"//[^\n]*", "", src)
-    start = src.index(name + "(", src.index("__global__"))
+    start = re.search(r"__launch_bounds__\([^)]*\)\s*" + name + r"\(", src).start()
     start = src.index("{", start)
     depth, i = 0, start
     while True:
@@ -46,3 +46,21 @@ def test_down_gemm_reads_the_plan_past_l1(name):
     """The table copy sits behind `if (MODE == 0) pdl_wait()`: in the down launch no wait precedes it."""
     body = kernel_body("gemm_tc5_ts.cuh", "expert_gemm_ts_kernel")
     assert loads(body, name) == (0, 1)
+
+
+@pytest.mark.parametrize("file,name", [
+    ("plan.cuh", "permute_kernel"),
+    ("route.cuh", "front_small_kernel"),
+    ("gemm_tc5_ts.cuh", "expert_gemm_ts_kernel"),
+    ("gemm_tc5_pair.cuh", "expert_gemm_pair_kernel"),
+    ("plan.cuh", "combine_kernel"),
+])
+def test_trigger_follows_the_wait(file, name):
+    """From the permute on: that a kernel has started then says that every kernel before its
+    predecessor is complete, which the reads ahead of the wait rest on."""
+    body = kernel_body(file, name)
+    calls = re.findall(r"pdl_(wait|trigger)\(\)", body)
+    assert "trigger" in calls
+    for i, c in enumerate(calls):
+        if c == "trigger":
+            assert i > 0 and calls[i - 1] == "wait", calls
