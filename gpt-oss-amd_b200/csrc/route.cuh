@@ -33,8 +33,11 @@
 // H + 1e-5f)) in IEEE float arithmetic, and o = weight * (scale * x) evaluated in
 // double and rounded to float once (src/run.cpp:306-319); that float is then
 // rounded to bf16, the block's input precision (src/hip/BLAS.hip:32-40).  Only the
-// order of the double additions differs (1e-16).
+// order of the double additions differs from the CPU engine's (1e-16); it is the same in
+// rows_to_bf16_kernel and front_small_kernel.
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace moe {
@@ -556,8 +559,8 @@ route_tc_kernel(const void* __restrict__ xv, int T, int H, const uint16_t* __res
 // Such a call is a chain of latencies, and a launch boundary costs more than the work
 // behind it.  One cluster of FRONT_CS CTAs: CTA r keeps the token rows' and the router's chunks
 // r, r + FRONT_CS, ... in shared memory as a whole (no ring: 6 of 45 chunks at H = 2880), CTA 0
-// adds the partial logits in rank order and selects, as in route_tc_kernel with a K split (the
-// same operations in the same order: the same bits), plans, and every CTA stores its
+// adds the partial logits in rank order and selects, as in route_tc_kernel with a K split of
+// eight (the same operations in the same order: the same bits), plans, and every CTA stores its
 // columns of the permuted rows from shared memory, so the bf16 rows are never re-read.
 constexpr int FRONT_CS = 8;
 constexpr int FRONT_MAX_T = 16;
@@ -613,23 +616,72 @@ front_small_kernel(const void* __restrict__ xv, int x_is_f32, const void* __rest
     pdl_trigger();
 
     if (rms_w) {
-        // the CPU engine's norm (rms_apply): float products summed in double, one warp per row
+        // The CPU engine's norm (rms_apply): float products summed in double.  One warp per row,
+        // with the additions of rows_to_bf16_kernel in its order, so that a row's bits are the
+        // same in a batch of any size: lane l adds what threads l, l + 32, ... add there, in a
+        // sum for each of those warps, and the eight sums are then added over the lanes in the
+        // same tree (a lane keeps half of them at each of the first three levels).  Against one
+        // sum per lane, which was another order (us per layer with the norm, 1 / 16 tokens): hidden
+        // 2880, 32 experts 44.0 / 130.3 -> 43.0 / 127.2; 2048 x 768, 128 experts 31.5 / 93.1 ->
+        // 31.7 / 93.6.
+        constexpr int RW = RCAST_THREADS / 32;
+        static_assert(RW == 8, "three levels of halving");
         for (int t = warp; t < T; t += RTHREADS / 32) {
             const float4* row = reinterpret_cast<const float4*>(static_cast<const float*>(xv) + (size_t)t * H);
-            double ss = 0.0;
-#pragma unroll 8
-            for (int v = lane; v < H / 4; v += 32) {
-                const float4 q = row[v];
-                ss += (double)(q.x * q.x);
-                ss += (double)(q.y * q.y);
-                ss += (double)(q.z * q.z);
-                ss += (double)(q.w * q.w);
-            }
+            double ss[RW];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-                ss += __shfl_xor_sync(0xffffffffu, ss, o);
-            if (lane == 0)
-                s_scale[t] = __fdiv_rn(1.0f, __fsqrt_rn((float)(ss / (double)H + (double)1e-5f)));
+            for (int w = 0; w < RW; w++)
+                ss[w] = 0.0;
+            // `n` groups of 32 vectors from v0 on; whole ones are loaded without a test, so that
+            // their loads are in flight together
+            auto add_groups = [&](auto n, auto whole, int v0) {
+                constexpr int N = decltype(n)::value;
+                float4 q[N];
+#pragma unroll
+                for (int i = 0; i < N; i++) {
+                    const int v = v0 + i * 32 + lane;
+                    q[i] = decltype(whole)::value || v < H / 4 ? row[v] : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+                for (int i = 0; i < N; i++) {
+                    ss[i % RW] += (double)(q[i].x * q[i].x);
+                    ss[i % RW] += (double)(q[i].y * q[i].y);
+                    ss[i % RW] += (double)(q[i].z * q[i].z);
+                    ss[i % RW] += (double)(q[i].w * q[i].w);
+                }
+            };
+            int v0 = 0;
+            if (2 * RCAST_THREADS <= H / 4) {
+                add_groups(std::integral_constant<int, 2 * RW>(), std::true_type(), 0);
+                v0 = 2 * RCAST_THREADS;
+            }
+#pragma unroll 1
+            for (; v0 + RCAST_THREADS <= H / 4; v0 += RCAST_THREADS)
+                add_groups(std::integral_constant<int, RW>(), std::true_type(), v0);
+            if (v0 < H / 4)
+                add_groups(std::integral_constant<int, RW>(), std::false_type(), v0);
+#pragma unroll
+            for (int keep = RW / 2; keep >= 1; keep >>= 1) {
+                const int o = 4 * keep;
+                const bool upper = (lane & o) != 0;
+#pragma unroll
+                for (int w = 0; w < keep; w++) {
+                    const double mine = upper ? ss[w + keep] : ss[w], give = upper ? ss[w] : ss[w + keep];
+                    ss[w] = mine + __shfl_xor_sync(0xffffffffu, give, o);
+                }
+            }
+            double part = ss[0];  // of warp (lane >> 2)
+            part += __shfl_xor_sync(0xffffffffu, part, 2);
+            part += __shfl_xor_sync(0xffffffffu, part, 1);
+            double tot = 0.0;
+#pragma unroll
+            for (int w = 0; w < RW; w++)
+                tot += __shfl_sync(0xffffffffu, part, 4 * w);
+            if (lane == 0) {
+                tot /= (double)H;
+                tot += (double)1e-5f;
+                s_scale[t] = __fdiv_rn(1.0f, __fsqrt_rn((float)tot));
+            }
         }
         __syncthreads();
     }

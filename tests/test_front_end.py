@@ -47,3 +47,45 @@ def test_front_end(H, I, E, K, T, form):
     compare(res, ref, K, f"{(H, I, E, K, T, form)}")
     assert np.abs(res["score"] - ref["router_score"]).max() < 1e-5
     assert list(np.bincount(ref["topk_i"].reshape(-1), minlength=E)) == res["counts"]
+
+
+def _row_at_a_rounding_edge(H):
+    """A row and the weight of its first column for which the order of the norm's additions
+    shows.  Sum of squares = a float midpoint m (the squares of columns 0 and 1) and twelve
+    squares of a quarter of m's ulp in double, in three groups of four: added to m one by one
+    they are all lost, group by group they are not.  Which of the two is stored moves the
+    scale by one ulp, and the weight puts column 0 on a bf16 rounding edge between the two."""
+    x = np.zeros(H, np.float32)
+    x[0], x[1] = np.float32(1109804032.0), np.float32(2.0**18)
+    for k in (32, 64, 96):  # float4 columns: one lane of a warp in both kernels
+        x[4 * k:4 * k + 4] = 8.0
+    m = float(x[0] * x[0]) + float(x[1] * x[1])
+    scales = [np.float32(1.0) / np.sqrt(np.float32((m + d) / H + float(np.float32(1e-5)))) for d in (0.0, 768.0)]
+    assert scales[0] != scales[1]
+    w = np.float32(0.99)
+    for _ in range(1 << 17):
+        rows = torch.tensor([float(np.float32(float(w) * (float(s) * float(x[0])))) for s in scales])
+        if rows.bfloat16()[0] != rows.bfloat16()[1]:
+            return torch.from_numpy(x), float(w)
+        w = np.nextafter(w, np.float32(2.0))
+    raise AssertionError("no weight found")
+
+
+@pytest.mark.parametrize("H,E,edge", [(512, 8, True), (512, 8, False), (2880, 32, False), (4160, 20, False)])
+@pytest.mark.parametrize("w_dtype", [torch.float32, torch.bfloat16])
+def test_a_row_does_not_depend_on_the_kernel_that_normed_it(H, E, edge, w_dtype):
+    """The first 16 rows in a batch of 16 (one launch) and of 17 (rows_to_bf16_kernel)."""
+    shape = pkg.MoEShape(hidden=H, intermediate=64, n_experts=E, top_k=2)
+    g = torch.Generator().manual_seed(H)
+    x = (3.0 * torch.randn(17, H, generator=g)).float()
+    w = (1.0 + 0.2 * torch.randn(H, generator=g)).float()
+    if edge:
+        x[0], w[0] = _row_at_a_rounding_edge(H)
+    with pkg.MoEEngine(shape, max_tokens=17) as eng:
+        eng.load_layer(0, synth.make_layer(shape, seed=H))
+        w = w.to(w_dtype).cuda()
+        a = [v.cpu() for v in eng.forward_norm(0, x[:16].cuda(), w, side=True)]
+        b = [v.cpu()[:16] for v in eng.forward_norm(0, x.cuda(), w, side=True)]
+        assert eng.device_status() == 0
+    for p, q in zip(a, b):
+        assert torch.equal(p, q)
