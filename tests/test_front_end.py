@@ -89,3 +89,36 @@ def test_a_row_does_not_depend_on_the_kernel_that_normed_it(H, E, edge, w_dtype)
         assert eng.device_status() == 0
     for p, q in zip(a, b):
         assert torch.equal(p, q)
+
+
+@pytest.mark.parametrize("H,I,E,K,T,launches", [
+    (576, 64, 20, 4, 1, 4),
+    (576, 64, 20, 4, 16, 4),
+    (2560, 64, 256, 2, 16, 4),  # the largest rows that fit shared memory with 256 experts
+    (2624, 64, 256, 2, 16, 6),  # one chunk more: the separate kernels
+    (4160, 64, 20, 4, 17, 6),   # rows above 4096 columns: weights fetched after the sum too
+])
+@pytest.mark.parametrize("w_dtype", [torch.float32, torch.bfloat16])
+def test_norm_and_residual_update(H, I, E, K, T, launches, w_dtype):
+    """forward_norm against the oracle with both weight types, the path it took, and the
+    engine's in-place x += MoE(rmsnorm(x)): one fp32 addition to the same result."""
+    shape = pkg.MoEShape(hidden=H, intermediate=I, n_experts=E, top_k=K)
+    lw = synth.make_layer(shape, seed=H + E + T)
+    g = torch.Generator().manual_seed(T)
+    x = (3.0 * torch.randn(T, H, generator=g)).float()
+    w = (1.0 + 0.2 * torch.randn(H, generator=g)).to(w_dtype)
+    x_bits = synth.bf16_bits(torch.from_numpy(oracle.rmsnorm(x.numpy(), w.float().numpy())))
+    ref = oracle_case(lw, x_bits)
+    with pkg.MoEEngine(shape, max_tokens=T) as eng:
+        eng.load_layer(0, lw)
+        out, sc, ti, tw = eng.forward_norm(0, x.cuda(), w.cuda(), side=True)
+        assert eng.last_launch_count() == launches
+        h = eng.last_intermediate(T)
+        stream = x.cuda()
+        eng.forward_norm(0, stream, w.cuda(), out=stream, accumulate=True)
+        torch.cuda.synchronize()
+        assert eng.device_status() == 0
+        res = {"out": out.cpu().numpy(), "topk_i": ti.cpu().numpy(), "topk_w": tw.cpu().numpy(),
+               "h_bits": h.cpu().numpy().view(np.uint16)}
+        assert torch.equal(stream.cpu(), x + out.cpu())
+    compare(res, ref, K, f"{(H, I, E, K, T, w_dtype)}")

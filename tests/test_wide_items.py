@@ -2,10 +2,11 @@
 changes or a tile is cut.  The oracle and its tolerances are those of test_gpu_parity.py."""
 import numpy as np
 import pytest
+import torch
 
 import gpt_oss_amd_b200 as pkg
 from gpt_oss_amd_b200 import capi, synth
-from parity_util import compare, oracle_case, run_gpu
+from parity_util import compare, compare_sampled, oracle_case, run_gpu
 
 pytestmark = pytest.mark.gpu
 
@@ -26,3 +27,34 @@ def test_wide_items(H, I, E, K, T, skew):
     ref = oracle_case(lw, x_bits)
     res = run_gpu(shape, lw, x_bits, capi.GEMM_TCGEN05)
     compare(res, ref, K, f"{(H, I, E, K, T, skew)}")
+
+
+@pytest.mark.parametrize("H,I,E,K,T", [
+    (2880, 2880, 32, 4, 777),   # 15 steps per item
+    (1088, 832, 64, 4, 1600),   # 6 and 5 steps, the last one cut in both launches
+])
+@pytest.mark.parametrize("skew", [False, True])
+def test_wide_items_reuse_their_rings(H, I, E, K, T, skew):
+    """CTAs that walk several items of many steps: every slot of the weight, activation and
+    tensor-memory rings, both accumulator sets and the parities of their barriers come round
+    again.  All rows against the cross-check GEMM (the same rounding points, another fp32
+    order: the bound of test_tcgen05_equals_mma_sync_at_prefill_size), a sample against the
+    oracle."""
+    shape = pkg.MoEShape(hidden=H, intermediate=I, n_experts=E, top_k=K)
+    lw = synth.make_layer(shape, seed=H + T, **(dict(zipf_s=1.1, zipf_gain=synth.ZIPF_GAIN_4X) if skew else {}))
+    x_bits = synth.make_tokens(T, H, seed=T)
+    res = run_gpu(shape, lw, x_bits, capi.GEMM_TCGEN05)  # asserts the status word
+    items = sum(-(-c // 128) for c in res["counts"])
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert 57 * E <= sum(res["counts"]) < 113 * E  # the rule that picks this form
+    for m_tiles, k in ((-(-2 * I // 128), H), (-(-H // 128), I)):
+        assert items * m_tiles >= 3 * sms and -(-k // 64 // 3) > 4
+    if skew:
+        assert max(res["counts"]) > 256  # more than two items of one expert
+    ref = run_gpu(shape, lw, x_bits, capi.GEMM_MMA_SYNC)
+    assert np.array_equal(ref["topk_i"], res["topk_i"])
+    d = ref["out"].astype(np.float64) - res["out"].astype(np.float64)
+    assert np.linalg.norm(d) / np.linalg.norm(ref["out"].astype(np.float64)) < 5e-4
+    sample = np.linspace(0, T - 1, 16).astype(int)
+    compare_sampled({k: res[k][sample] for k in ("out", "topk_i", "topk_w", "h_bits")}, lw, x_bits[sample],
+                    lw.w_router, lw.b_router, K, f"{(H, I, E, K, T, skew)}")
