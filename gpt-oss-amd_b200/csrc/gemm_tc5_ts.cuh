@@ -21,9 +21,10 @@
 // with the decoded weights as the UMMA A operand IN TENSOR MEMORY (tcgen05.mma
 // "TS" form: lane = weight row, one 32-bit column = two consecutive bf16 of K,
 // written by the decode warps with tcgen05.st straight from registers) and the
-// token rows as the B operand in shared memory (N = 32 or 64, a TMA box).  The
-// tensor work is small (the four MMAs of a 128 x 32 x 64 chunk issue in ~100
-// cycles), shared memory carries only the packed bytes and the small activation tile.
+// token rows as the B operand in shared memory (N = the item's rows rounded up to a
+// multiple of 16, a TMA box).  The tensor work is small (the four MMAs of a 128 x 32 x 64
+// chunk issue in ~100 cycles), shared memory carries only the packed bytes and the small
+// activation tile.
 //
 // One persistent CTA per SM walks work items (expert, 128-row weight tile, tile
 // of up to 64 token rows, or 128 in the wide variant: medium batches, where 64-row items
@@ -36,12 +37,14 @@
 // MMA-issuing warp needs ~25 cycles per tcgen05.mma at N = 32 (the tensor pipe's
 // own rate) but ~800 cycles per step around them -- one barrier test, one commit
 // and a little bookkeeping, each a round trip through a memory pipe that sixteen
-// decode warps keep busy -- and it is the only warp that can issue them.  Rings:
+// decode warps keep busy -- and it is the only warp that can issue them.  Rings (of the
+// narrow form; Config holds the sizes of both):
 //   W ring   packed MXFP4 steps in shared memory (bulk copies; covers HBM latency)
 //   A ring   SA = 2 slots of 192 tensor-memory columns (decoded weights)
 //   B ring   activation tiles in shared memory (one 3-d TMA box per step, no
 //            multicast), handed out in units of 24 KB: a step of an item with up to
-//            32 token rows takes one unit, with up to 64 rows two
+//            32 token rows takes one unit, with up to 64 rows two.  (Wide: three slots
+//            of 48 KB, one 2-d box per chunk)
 // and NB barrier pairs indexed by the step number: full[i % NB] collects the
 // decode warps' arrivals and the TMA bytes of step i, empty[i % NB] is signalled
 // by tcgen05.commit when the MMAs of step i are done.
@@ -142,14 +145,14 @@ struct TileInfo {
     int e;        // local expert
     int mt;       // 128-row weight tile
     int row0;     // first token row of the item
-    int valid_n;  // token rows of the item (1..64)
+    int valid_n;  // token rows of the item (1..64, Wide 1..128)
     int n_mma;    // rows the MMA computes and the TMA box holds (a multiple of 16)
 };
 
 struct TileTables {
     const int* off;         // [E + 1]
     const int* cnt;         // [E]
-    const int* tile_start;  // [E + 1]  prefix of ceil(cnt / BN)
+    const int* tile_start;  // [E + 1]  prefix of ceil(cnt / C::BN)
 };
 
 // Items ordered [expert][weight tile][token tile]: the token tiles that share

@@ -235,7 +235,12 @@ constexpr int FRONT_MAX_SMEM = 220 * 1024;
 // items.  Measured (hidden 2880, us per layer, 64-row items / 128-row items / CTA pairs):
 // 32 experts, 384 tokens (48 rows) 187 / 200 / -, 512 (64 rows) 234 / 220 / -, 777 (97 rows)
 // - / 255 / 303; 128 experts, 3001 tokens (94 rows) - / 990 / 1104, 4096 (128 rows) -
-// / 1329 / 1206.
+// / 1329 / 1206.  The rule sees only the average, but skewed routing keeps the order (means of
+// runs in turn, busiest expert 4 / 7 times the average at 32 experts, 13 / 27 times at 128):
+// 32 experts, 464 tokens (58 rows), 64-row / 128-row items 210 / 211 and 237 / 232; 777 tokens,
+// 128-row items / CTA pairs 258 / 305 and 277 / 320; 128 experts, 3001 tokens 1102 / 1183 and
+// 1054 / 1101; 2048 x 768, 128 experts top-8, 1500 tokens (11 and 16 times) 292 / 308 and
+// 268 / 297.
 constexpr int SMALL_MAX_ROWS_PER_EXPERT = 56;
 constexpr int WIDE_MAX_ROWS_PER_EXPERT = 112;
 
@@ -607,8 +612,9 @@ int permute_split(moe_b200_handle h, int nblk, int n_assign) {
 // Token rows per GEMM tile for a call that has `rows` rows spread over the local
 // experts; the tile tables are built for it and it selects the kernel: few rows per
 // expert (bound by streaming the weights) -> the single-CTA kernel with the decoded
-// weights in tensor memory, 64 token rows per tile; otherwise CTA pairs and 256
-// token rows per tile.  Any choice is correct for any distribution of rows.
+// weights in tensor memory, 64 token rows per tile; a medium number -> the same kernel
+// with 128 token rows per tile; otherwise CTA pairs and 256 token rows per tile.  Any
+// choice is correct for any distribution of rows.
 int pick_bn(moe_b200_handle h, int rows) {
 #ifdef MOE_B200_TEST_AIDS
     if (h->cfg.gemm_impl == MOE_B200_GEMM_MMA_SYNC)
@@ -986,9 +992,9 @@ moe_b200_status moe_b200_load_experts_file(moe_b200_handle h, const char* path, 
 
 namespace {
 
-// The block.  With `rms_w` the input is the fp32 residual stream: the router kernel
-// applies the norm, writes the normalised rows as bf16 into the handle's workspace
-// and the permute kernel gathers from there.
+// The block.  With `rms_w` the input is the fp32 residual stream: rows_to_bf16_kernel applies
+// the norm and writes the normalised rows as bf16 into the handle's workspace, where the
+// router and the permute kernel read them (up to 16 tokens: front_small_kernel does all of it).
 moe_b200_status forward_impl(moe_b200_handle h, int layer, const void* t, int t_dtype, const void* rms_w,
                              int rms_w_dtype, int n_tokens, float* out, int accumulate,
                              float* router_score_out, int* topk_i_out, float* topk_w_out,

@@ -19,7 +19,7 @@ struct TensorMaps {
     // its MMA computes and no more: at the decode rate the activations of a step weigh as much as
     // its packed weights on the way from L2.  Against boxes of 32, 64 and 128 rows (us per
     // layer, hidden 2880): 200 tokens x 128 experts 521 -> 479, 128 tokens x 32 147 -> 135,
-    // 3001 x 128 991 -> 945, 16384 x 128 3468 -> 3356.
+    // 3001 x 128 991 -> 945; large batches within the spread of their runs.
     CUtensorMap box[8];
     // the same rows seen as [chunk of 64 columns][row][64 columns]: boxes of 16 (i + 1)
     // rows x STEP_CHUNKS chunks, so that one copy brings the activation tiles of a whole step
