@@ -425,11 +425,20 @@ cudaError_t launch_front_nt(moe_b200_handle h, const LayerWeights& lw, const voi
 }
 
 // One routing block and one GPU.  At 17 tokens the copies of the permuted rows would already
-// want more than one cluster; expert parallelism places rows on other GPUs.
-bool front_fits(moe_b200_handle h, int T) {
+// want more than one cluster; expert parallelism places rows on other GPUs.  With the norm, long
+// rows go to the separate kernels when a warp would have two of them: all eight CTAs norm all
+// rows, a warp each, and from 4096 columns on the second row costs more than the launches it
+// saves (us per layer at 16 tokens, this kernel / the separate ones; hidden x intermediate,
+// experts, top-k: 2048 x 768, 128, 8 92.8 / 101.5; 2880 x 2880, 32, 4 127.2 / 124.0; 2880 x 2880,
+// 128, 4 201 / 207; 3072 x 1024, 128, 8 144.0 / 144.7; 4096 x 1024, 64, 8 138.0 / 135.2; 5120 x 1024,
+// 128, 4 153 / 154; 6144 x 1024, 32, 4 126 / 113; 8192 x 1024, 32, 4 160 / 142).
+constexpr int FRONT_NORM_LONG_ROW = 4096;
+bool front_fits(moe_b200_handle h, int T, bool norm) {
     const int nt = ceil_div(h->cfg.n_experts, 32), H = h->cfg.hidden_dim;
     const size_t bytes = nt <= 1 ? front_smem_bytes<1>(H) : nt <= 2 ? front_smem_bytes<2>(H)
                          : nt <= 4 ? front_smem_bytes<4>(H) : front_smem_bytes<8>(H);
+    if (norm && T > RTHREADS / 32 && H >= FRONT_NORM_LONG_ROW)
+        return false;
     return h->cfg.ep_size == 1 && h->cfg.device < MAX_DEVICES && T > 0 && T <= FRONT_MAX_T &&
            H <= 4 * RCAST_THREADS * RCAST_MAX_VEC && bytes <= (size_t)FRONT_MAX_SMEM;
 }
@@ -1045,7 +1054,7 @@ moe_b200_status forward_impl(moe_b200_handle h, int layer, const void* t, int t_
     if (!h->prof_external)
         h->prof_call = (h->prof_next < h->prof_armed) ? h->prof_next++ : -1;
 
-    const bool front = front_fits(h, T);
+    const bool front = front_fits(h, T, rms_w != nullptr);
     if (front) {
         prof_mark(h, MOE_B200_STAGE_ROUTE, true, s);
         CU_TRY(h, launch_front(h, lw, t, (int)(t_dtype == MOE_B200_DTYPE_F32), rms_w,

@@ -71,21 +71,24 @@ def _row_at_a_rounding_edge(H):
     raise AssertionError("no weight found")
 
 
-@pytest.mark.parametrize("H,E,edge", [(512, 8, True), (512, 8, False), (2880, 32, False), (4160, 20, False)])
+@pytest.mark.parametrize("H,E,T,edge", [(512, 8, 16, True), (512, 8, 16, False), (2880, 32, 16, False),
+                                        (4160, 20, 8, False)])
 @pytest.mark.parametrize("w_dtype", [torch.float32, torch.bfloat16])
-def test_a_row_does_not_depend_on_the_kernel_that_normed_it(H, E, edge, w_dtype):
-    """The first 16 rows in a batch of 16 (one launch) and of 17 (rows_to_bf16_kernel)."""
+def test_a_row_does_not_depend_on_the_kernel_that_normed_it(H, E, T, edge, w_dtype):
+    """The first T rows in a batch of T (one launch) and of T + 1 (rows_to_bf16_kernel)."""
     shape = pkg.MoEShape(hidden=H, intermediate=64, n_experts=E, top_k=2)
     g = torch.Generator().manual_seed(H)
-    x = (3.0 * torch.randn(17, H, generator=g)).float()
+    x = (3.0 * torch.randn(T + 1, H, generator=g)).float()
     w = (1.0 + 0.2 * torch.randn(H, generator=g)).float()
     if edge:
         x[0], w[0] = _row_at_a_rounding_edge(H)
-    with pkg.MoEEngine(shape, max_tokens=17) as eng:
+    with pkg.MoEEngine(shape, max_tokens=T + 1) as eng:
         eng.load_layer(0, synth.make_layer(shape, seed=H))
         w = w.to(w_dtype).cuda()
-        a = [v.cpu() for v in eng.forward_norm(0, x[:16].cuda(), w, side=True)]
-        b = [v.cpu()[:16] for v in eng.forward_norm(0, x.cuda(), w, side=True)]
+        a = [v.cpu() for v in eng.forward_norm(0, x[:T].cuda(), w, side=True)]
+        assert eng.last_launch_count() == 4
+        b = [v.cpu()[:T] for v in eng.forward_norm(0, x.cuda(), w, side=True)]
+        assert eng.last_launch_count() == 6
         assert eng.device_status() == 0
     for p, q in zip(a, b):
         assert torch.equal(p, q)
@@ -94,6 +97,12 @@ def test_a_row_does_not_depend_on_the_kernel_that_normed_it(H, E, edge, w_dtype)
 @pytest.mark.parametrize("H,I,E,K,T,launches", [
     (576, 64, 20, 4, 1, 4),
     (576, 64, 20, 4, 16, 4),
+    # Long rows, with an intermediate of 256: the parity rule allows one rounding flip of h in
+    # 1000 elements, about 1 in 2000 is expected at this length, and 9 x 4 x 64 elements are too
+    # few to tell the two apart (3 flips against a limit of 2.3).
+    (4096, 256, 20, 4, 8, 4),   # a long row for every warp
+    (4096, 256, 20, 4, 9, 6),   # one more: the separate kernels
+    (4032, 256, 20, 4, 16, 4),  # the longest rows of which a warp takes two
     (2560, 64, 256, 2, 16, 4),  # the largest rows that fit shared memory with 256 experts
     (2624, 64, 256, 2, 16, 6),  # one chunk more: the separate kernels
     (4160, 64, 20, 4, 17, 6),   # rows above 4096 columns: weights fetched after the sum too
