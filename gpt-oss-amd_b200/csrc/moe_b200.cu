@@ -1068,9 +1068,10 @@ moe_b200_status forward_impl(moe_b200_handle h, int layer, const void* t, int t_
             // bf16 rows every later kernel reads: one pass, norm folded in when asked
             if (H > 4 * RCAST_THREADS * RCAST_MAX_VEC)
                 return fail(h, MOE_B200_ERR_UNSUPPORTED, "fp32 input is supported up to hidden_dim 8192");
-            CU_TRY(h, launch_kernel(pdl, rows_to_bf16_kernel, dim3(T), dim3(RCAST_THREADS), 0, s,
-                                    static_cast<const float*>(t), T, H, rms_w,
-                                    (int)(rms_w_dtype == MOE_B200_DTYPE_F32), h->xn));
+            const auto cast = T <= RCAST_EARLY_BLOCKS_PER_SM * h->n_sms ? rows_to_bf16_kernel<true>
+                                                                        : rows_to_bf16_kernel<false>;
+            CU_TRY(h, launch_kernel(pdl, cast, dim3(T), dim3(RCAST_THREADS), 0, s, static_cast<const float*>(t),
+                                    T, H, rms_w, (int)(rms_w_dtype == MOE_B200_DTYPE_F32), h->xn));
             h->last_launches++;
             t = h->xn;
             t_dtype = MOE_B200_DTYPE_BF16;

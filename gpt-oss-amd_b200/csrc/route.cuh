@@ -166,8 +166,13 @@ __device__ __forceinline__ float rms_apply(float x, float w, float scale) {
 // between the sum of squares and the scaling (H <= 8192).
 constexpr int RCAST_THREADS = 256;
 constexpr int RCAST_MAX_VEC = 8;  // float4 per thread: H <= 8192
+// EARLY: the first norm weights are fetched with the row, not after the sum over it (rows of up
+// to 4096 columns: all of them).  It saves a load latency and costs 16 registers, that is
+// one of four blocks per SM, so it is for batches of one wave (RCAST_EARLY_BLOCKS_PER_SM).
 constexpr int RCAST_EARLY_VEC = 4;
+constexpr int RCAST_EARLY_BLOCKS_PER_SM = 3;
 
+template <bool EARLY>
 __global__ void __launch_bounds__(RCAST_THREADS)
 rows_to_bf16_kernel(const float* __restrict__ x, int T, int H, const void* __restrict__ rms_w,
                     int rms_w_is_f32, uint16_t* __restrict__ out) {
@@ -193,10 +198,8 @@ rows_to_bf16_kernel(const float* __restrict__ x, int T, int H, const void* __res
         return make_float4(__uint_as_float(wq.x << 16), __uint_as_float(wq.x & 0xFFFF0000u),
                            __uint_as_float(wq.y << 16), __uint_as_float(wq.y & 0xFFFF0000u));
     };
-    // the first weights are fetched with the row, not after the sum over it (rows of up to
-    // 4096 columns: all of them)
     float4 wv[RCAST_EARLY_VEC];
-    if (rms_w) {
+    if (EARLY && rms_w) {
 #pragma unroll
         for (int i = 0; i < RCAST_EARLY_VEC; i++) {
             const int k = tid + i * RCAST_THREADS;
@@ -239,7 +242,7 @@ rows_to_bf16_kernel(const float* __restrict__ x, int T, int H, const void* __res
         if (k < nvec) {
             float4 q = v[i];
             if (rms_w) {
-                const float4 w = i < RCAST_EARLY_VEC ? wv[i] : weight(k);
+                const float4 w = EARLY && i < RCAST_EARLY_VEC ? wv[i] : weight(k);
                 q.x = rms_apply(q.x, w.x, scale), q.y = rms_apply(q.y, w.y, scale);
                 q.z = rms_apply(q.z, w.z, scale), q.w = rms_apply(q.w, w.w, scale);
             }
