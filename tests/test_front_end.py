@@ -131,3 +131,23 @@ def test_norm_and_residual_update(H, I, E, K, T, launches, w_dtype):
                "h_bits": h.cpu().numpy().view(np.uint16)}
         assert torch.equal(stream.cpu(), x + out.cpu())
     compare(res, ref, K, f"{(H, I, E, K, T, w_dtype)}")
+
+
+@pytest.mark.parametrize("H", [576, 4160])
+def test_norm_with_early_and_late_weights(H):
+    """rows_to_bf16_kernel fetches its norm weights ahead of the sum up to three rows per SM: the
+    last batch that does and the first that does not give the same bits (both are 28 routing
+    blocks on 148 SMs, so the router splits K alike)."""
+    T = 3 * torch.cuda.get_device_properties(0).multi_processor_count
+    shape = pkg.MoEShape(hidden=H, intermediate=64, n_experts=20, top_k=2)
+    g = torch.Generator().manual_seed(H)
+    x = (3.0 * torch.randn(T + 1, H, generator=g)).float().cuda()
+    w = (1.0 + 0.2 * torch.randn(H, generator=g)).float().cuda()
+    with pkg.MoEEngine(shape, max_tokens=T + 1) as eng:
+        eng.load_layer(0, synth.make_layer(shape, seed=H))
+        early = eng.forward_norm(0, x[:T], w, side=True)
+        late = eng.forward_norm(0, x, w, side=True)
+        torch.cuda.synchronize()
+        assert eng.device_status() == 0
+    for p, q in zip(early, late):
+        assert torch.equal(p, q[:T])
