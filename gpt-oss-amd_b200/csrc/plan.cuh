@@ -260,22 +260,27 @@ combine_kernel(const float* __restrict__ y, int T, int H, int K, const int* __re
                const float* __restrict__ topk_w, const int* __restrict__ slot_of,
                float* __restrict__ out, int accumulate, const int* __restrict__ wait_flags, int G,
                int seq, int* __restrict__ status) {
-    // the routing is two kernels old and more: complete before this kernel starts, and read past
-    // L1 because this kernel has not waited yet (ld_l2)
+    // The routing is two kernels old and more: complete before this kernel starts, and read past
+    // L1 because this kernel has not waited yet (ld_l2).  One warp reads it for the block: eight
+    // warps asking L2 for the same words cost 8000 short rows 2 us of 31.
     const int t = blockIdx.x;
+    __shared__ int s_ex[8], s_sl[8];
+    __shared__ float s_wt[8];
+    if (threadIdx.x < 8) {
+        const int k = threadIdx.x;
+        const bool used = k < K && t < T;
+        s_ex[k] = used ? ld_l2(topk_i + (size_t)t * K + k) : 0x7fffffff;
+        s_sl[k] = used ? ld_l2(slot_of + (size_t)t * K + k) : 0;
+        s_wt[k] = used ? ld_l2(topk_w + (size_t)t * K + k) : 0.f;
+    }
+    __syncthreads();
     int ex[8], sl[8];
     float wt[8];
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-        if (k < K && t < T) {
-            ex[k] = ld_l2(topk_i + (size_t)t * K + k);
-            sl[k] = ld_l2(slot_of + (size_t)t * K + k);
-            wt[k] = ld_l2(topk_w + (size_t)t * K + k);
-        } else {
-            ex[k] = 0x7fffffff;
-            sl[k] = 0;
-            wt[k] = 0.f;
-        }
+        ex[k] = s_ex[k];
+        sl[k] = s_sl[k];
+        wt[k] = s_wt[k];
     }
     // sort by expert index (K <= 8): odd-even transposition network on registers
 #pragma unroll
