@@ -301,8 +301,8 @@ moe_b200_status moe_b200_last_expert_counts(moe_b200_handle h, int* counts);
 /* One kernel may do the work of several stages; it counts in the first of them
  * and the others read the few microseconds of an empty event pair.  On one GPU
  * the PERMUTE kernel also plans for up to 32 routing blocks (512 tokens), and
- * for up to 16 tokens one kernel in ROUTE does the fp32 conversion or norm,
- * the routing, the plan and the gather. */
+ * for up to 16 tokens (fewer with the norm and long rows) one kernel in ROUTE
+ * does the fp32 conversion or norm, the routing, the plan and the gather. */
 #define MOE_B200_STAGE_ROUTE 0    /* fp32 -> bf16 (norm), router GEMM, top-k, softmax */
 #define MOE_B200_STAGE_PLAN 1     /* offsets, tile table                     */
 #define MOE_B200_STAGE_PERMUTE 2  /* row gather into expert order            */
