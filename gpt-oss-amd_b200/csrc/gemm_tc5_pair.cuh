@@ -336,73 +336,59 @@ expert_gemm_pair_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* 
         bool ok = true;
         if (!leader) {
             // ------------------------- peer: forward full[i] to the leader -------
-            int it = 0;
-            for (int tile = pair_id; ok && tile < total_tiles; tile += n_pairs, ++it) {
-                for (int ks = 0; ks < k_stages; ks++) {
-                    ok = mbar_wait_hot(bar_full(nb), ph, status, DS_TIMEOUT_FULL_A, abort_flag);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok)
-                        break;
-                    if (elect_one_sync())
+            if (elect_one_sync()) {
+                for (int tile = pair_id; ok && tile < total_tiles; tile += n_pairs) {
+                    for (int ks = 0; ks < k_stages; ks++) {
+                        ok = mbar_wait_hot(bar_full(nb), ph, status, DS_TIMEOUT_FULL_A, abort_flag);
+                        if (!ok)
+                            break;
                         mbar_arrive_remote(bar_full(nb), 0);
-                    RING_ADVANCE(nb, ph, NB);
+                        RING_ADVANCE(nb, ph, NB);
+                    }
                 }
             }
-        } else {
+        } else if (elect_one_sync()) {
             // ------------------------- leader: MMA issuer --------------------------
-            // The whole warp runs the loop with no lane-divergent code but the elected
-            // issue; the barrier of the NEXT step is tested before the MMAs of this
-            // step are issued, so that its latency overlaps the issue.
+            // One thread runs the loop: each instruction between two steps delays the next MMAs, and votes,
+            // elections and reconvergence of a whole warp were most of them (a whole warp, with the barrier
+            // of the next step tested ahead, against this; us per layer, hidden 2880: 32 experts, 1000 tokens
+            // 306 -> 299, 2048 tokens 448 -> 441, 8192 skewed 1325 -> 1317; 128 experts, 4500 tokens
+            // 1092 -> 1085).
             int it = 0;
-            bool ready = false;  // full[nb] already seen complete for phase ph
             for (int tile = pair_id; ok && tile < total_tiles; tile += n_pairs, ++it) {
                 const TileInfo ti = decode_tile(tile, m_pairs, tt, E);
                 const int set = it % SETS, round = it / SETS;
                 ok = mbar_wait(bar_tmem_empty(set), (uint32_t)(round & 1) ^ 1u, status,
                                DS_TIMEOUT_TMEM_EMPTY, abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
                 if (!ok)
                     break;
                 tc_fence_after();  // the epilogues' tcgen05.ld of this set came before
                 const uint32_t d_tmem = tmem_base + (uint32_t)(set * BN);
                 const uint32_t idesc = make_idesc2(ti.n_mma);
                 for (int ks = 0; ks < k_stages; ks++) {
-                    if (!ready) {
-                        ok = mbar_wait_hot(bar_full(nb), ph, status, DS_TIMEOUT_FULL_A, abort_flag);
-                        ok = __all_sync(0xffffffffu, ok);
-                        if (!ok)
-                            break;
-                    }
-                    if (lane == 0)
-                        TRACE(it * k_stages + ks, 4);
-                    int nb_next = nb;
-                    uint32_t ph_next = ph;
-                    RING_ADVANCE(nb_next, ph_next, NB);
-                    const uint32_t peek = mbar_try_wait(bar_full(nb_next), ph_next);
+                    ok = mbar_wait_hot(bar_full(nb), ph, status, DS_TIMEOUT_FULL_A, abort_flag);
+                    if (!ok)
+                        break;
+                    TRACE(it * k_stages + ks, 4);
                     const uint64_t a_desc = make_sw128_desc(smem_u32(a_ring + sa * A_SLOT_BYTES));
                     const uint64_t b_desc = make_sw128_desc(smem_u32(b_ring + sb * B_SLOT_BYTES));
-                    if (elect_one_sync()) {
 #pragma unroll
-                        for (int kk = 0; kk < KSTAGE / 16; kk++)
-                            umma2_bf16(d_tmem, a_desc + (uint64_t)(kk * 2), b_desc + (uint64_t)(kk * 2),
-                                       idesc, (ks | kk) != 0 ? 1u : 0u);
-                        umma2_commit_both(bar_empty(nb));  // frees the slots of both CTAs
-                    }
-                    if (lane == 0)
-                        TRACE(it * k_stages + ks, 5);
-                    ready = __all_sync(0xffffffffu, peek != 0);
-                    nb = nb_next;
-                    ph = ph_next;
+                    for (int kk = 0; kk < KSTAGE / 16; kk++)
+                        umma2_bf16(d_tmem, a_desc + (uint64_t)(kk * 2), b_desc + (uint64_t)(kk * 2), idesc,
+                                   (ks | kk) != 0 ? 1u : 0u);
+                    umma2_commit_both(bar_empty(nb));  // frees the slots of both CTAs
+                    TRACE(it * k_stages + ks, 5);
+                    RING_ADVANCE(nb, ph, NB);
                     if (++sa == SA)
                         sa = 0;
                     if (++sb == SB)
                         sb = 0;
                 }
-                if (ok && elect_one_sync())
+                if (ok)
                     umma2_commit_both(bar_tmem_full(set));
-                __syncwarp();
             }
         }
+        __syncwarp();
     } else if (warp < EPI_WARP0) {
         // ------------------------------ MXFP4 decode --------------------------
         // Four groups of 4 warps; group g decodes the pipeline steps g, g + 4, ...
