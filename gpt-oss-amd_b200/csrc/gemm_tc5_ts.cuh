@@ -51,7 +51,7 @@
 //
 // Warp roles:
 //   warp 0      W producer          warp 1   B producer (TMA)
-//   warp 2      allocates tensor memory, issues tcgen05.mma, commits
+//   warp 2      allocates tensor memory; one thread issues tcgen05.mma and commits
 //   next 16     decode packed MXFP4 -> bf16 -> tensor memory: two groups of eight
 //               warps, group g decodes steps g, g + 2, ...; two warps share a
 //               quarter of the rows, one takes the even chunks of the step, the
@@ -378,46 +378,43 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
         }
     } else if (warp == MMA_WARP) {
         // ------------------------------ MMA issuer ----------------------------
-        // The whole warp runs the loop with no lane-divergent code but the elected issue.
-        // This warp's chain per step (one barrier test, the MMAs, one commit, a little
-        // bookkeeping) is what paces the kernel once the rings are deep enough -- the
-        // operands of a step are ready thousands of cycles before it gets to them -- so
-        // it carries nothing else: one plain wait per step, no look-ahead test.
-        int sa = 0, bu = 0, nb = 0;  // step i: A slot i % SA, barriers i % NB, B units as the producer hands them out
-        uint32_t ph = 0;             // (i / NB) & 1
-        bool ok = true;
-        int it = 0;
-        for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++it) {
-            const TileInfo ti = decode_tile<C>(tile, m_tiles, tt, E);
-            const int set = it % SETS, round = it / SETS;
-            ok = mbar_wait(bar_tmem_empty(set), (uint32_t)(round & 1) ^ 1u, status,
-                           DS_TIMEOUT_TMEM_EMPTY, abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok)
-                break;
-            tc_fence_after();  // the epilogue's tcgen05.ld of this set came before
-            if (lane == 0)
-                TRACE(it * n_steps, 12);
-            const uint32_t d_tmem = tmem_base + (uint32_t)(set * C::BN);
-            const uint32_t idesc = make_idesc(ti.n_mma);
-            const int need = C::UNITS ? (ti.n_mma + 31) >> 5 : 1;  // B units per step
-            const uint32_t sub_step = (uint32_t)ti.n_mma * 8u;  // one chunk's tile in descriptor units of 16 bytes
-            for (int st = 0; st < n_steps; st++) {
-                ok = mbar_wait_hot(bar_full(nb), ph, status, DS_TIMEOUT_FULL_A, abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
+        // ONE thread runs the loop.  Its chain per step (one barrier test, the MMAs, one commit, a
+        // little bookkeeping) is what paces the kernel once the rings are deep enough, and each of its
+        // instructions waits for issue slots that the decode warps of its scheduler want nearly every
+        // cycle.  So no votes, elections or reconvergence between the MMAs (a whole warp with an elected
+        // issue against this, us per layer, hidden 2880: 32 experts, 1 token with the norm 44.8 -> 43.7,
+        // 16 tokens 124.1 -> 119.3, 64 tokens 133.5 -> 128.5, 256 tokens 140.7 -> 136; 128 experts,
+        // 200 tokens 446 -> 428).
+        if (elect_one_sync()) {
+            int sa = 0, bu = 0, nb = 0;  // step i: A slot i % SA, barriers i % NB, B units as the producer hands them out
+            uint32_t ph = 0;             // (i / NB) & 1
+            bool ok = true;
+            int it = 0;
+            for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++it) {
+                const TileInfo ti = decode_tile<C>(tile, m_tiles, tt, E);
+                const int set = it % SETS, round = it / SETS;
+                ok = mbar_wait(bar_tmem_empty(set), (uint32_t)(round & 1) ^ 1u, status, DS_TIMEOUT_TMEM_EMPTY,
+                               abort_flag);
                 if (!ok)
                     break;
-                if (lane == 0)
+                tc_fence_after();  // the epilogue's tcgen05.ld of this set came before
+                TRACE(it * n_steps, 12);
+                const uint32_t d_tmem = tmem_base + (uint32_t)(set * C::BN);
+                const uint32_t idesc = make_idesc(ti.n_mma);
+                const int need = C::UNITS ? (ti.n_mma + 31) >> 5 : 1;  // B units per step
+                const uint32_t sub_step = (uint32_t)ti.n_mma * 8u;  // one chunk's tile in descriptor units of 16 bytes
+                for (int st = 0; st < n_steps; st++) {
+                    ok = mbar_wait_hot(bar_full(nb), ph, status, DS_TIMEOUT_FULL_A, abort_flag);
+                    if (!ok)
+                        break;
                     TRACE(it * n_steps + st, 4);
-                tc_fence_after();  // the decode warps' tcgen05.st of this step came before
-                const uint32_t a_tmem = tmem_base + (uint32_t)(C::TMEM_A0 + sa * C::A_SLOT_COLS);
-                if (C::UNITS && need == 2 && (bu & 1))
-                    bu = (bu + 1) & (C::SB - 1);
-                const uint64_t b_desc = make_sw128_desc(smem_u32(b_ring + bu * C::B_SLOT_BYTES));
-                const uint32_t b_lo = (uint32_t)b_desc, b_hi = (uint32_t)(b_desc >> 32);
-                const int nch = min(C::CS, k_stages - st * C::CS);
-                if (elect_one_sync()) {
-                    TRACE(it * n_steps + st, 13);
+                    tc_fence_after();  // the decode warps' tcgen05.st of this step came before
+                    const uint32_t a_tmem = tmem_base + (uint32_t)(C::TMEM_A0 + sa * C::A_SLOT_COLS);
+                    if (C::UNITS && need == 2 && (bu & 1))
+                        bu = (bu + 1) & (C::SB - 1);
+                    const uint64_t b_desc = make_sw128_desc(smem_u32(b_ring + bu * C::B_SLOT_BYTES));
+                    const uint32_t b_lo = (uint32_t)b_desc, b_hi = (uint32_t)(b_desc >> 32);
+                    const int nch = min(C::CS, k_stages - st * C::CS);
 #pragma unroll
                     for (int j = 0; j < C::CS; j++) {
                         if (j < nch) {
@@ -428,20 +425,18 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                                              (st | j | kk) != 0 ? 1u : 0u);
                         }
                     }
-                    TRACE(it * n_steps + st, 14);
                     umma_commit(bar_empty(nb));  // frees both slots when these MMAs have read them
-                }
-                if (lane == 0)
                     TRACE(it * n_steps + st, 5);
-                RING_ADVANCE(nb, ph, C::NB);
-                if (++sa == C::SA)
-                    sa = 0;
-                bu = next_unit(bu, need);
+                    RING_ADVANCE(nb, ph, C::NB);
+                    if (++sa == C::SA)
+                        sa = 0;
+                    bu = next_unit(bu, need);
+                }
+                if (ok)
+                    umma_commit(bar_tmem_full(set));
             }
-            if (ok && elect_one_sync())
-                umma_commit(bar_tmem_full(set));
-            __syncwarp();
         }
+        __syncwarp();
     } else if (warp < EPI_WARP0) {
         // ------------------------------ MXFP4 decode --------------------------
         // Group g decodes the pipeline steps g, g + G, ...  A warp may write the
