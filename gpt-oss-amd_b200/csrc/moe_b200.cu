@@ -1179,17 +1179,20 @@ moe_b200_status forward_impl(moe_b200_handle h, int layer, const void* t, int t_
         // peer mode launches it for T == 0 as well: the wait inside is what orders this
         // rank's next call behind the peers' reads of this one
         prof_mark(h, MOE_B200_STAGE_COMBINE, true, s);
+        // the combine stores the routing for the caller too; a pointer that no int or float store may
+        // take gets a copy behind it
+        auto word_aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 3u) == 0; };
+        int* const ti_direct = word_aligned(topk_i_out) ? topk_i_out : nullptr;
+        float* const tw_direct = word_aligned(topk_w_out) ? topk_w_out : nullptr;
         const int combine_split = T <= 2 * h->n_sms && !peer_mode ? ceil_div(H / 4, 256) : 1;
-        CU_TRY(h, launch_kernel(pdl, combine_kernel, dim3(T > 0 ? T : 1, combine_split), dim3(256), 0, s, y_for_combine, T, H,
-                                K, h->topk_i, h->topk_w, h->slot_of, out, accumulate, combine_wait, c.ep_size,
-                                seq, h->status));
+        CU_TRY(h, launch_kernel(pdl, ti_direct || tw_direct ? combine_kernel<true> : combine_kernel<false>,
+                                dim3(T > 0 ? T : 1, combine_split), dim3(256), 0, s, y_for_combine, T, H, K, h->topk_i, h->topk_w, h->slot_of, out, accumulate, ti_direct, tw_direct,
+                                combine_wait, c.ep_size, seq, h->status));
         prof_mark(h, MOE_B200_STAGE_COMBINE, false, s);
         h->last_launches++;
-    }
-    if (T > 0) {
-        if (topk_i_out)
+        if (T > 0 && topk_i_out != ti_direct)
             CU_TRY(h, cudaMemcpyAsync(topk_i_out, h->topk_i, (size_t)T * K * 4, cudaMemcpyDeviceToDevice, s));
-        if (topk_w_out)
+        if (T > 0 && topk_w_out != tw_direct)
             CU_TRY(h, cudaMemcpyAsync(topk_w_out, h->topk_w, (size_t)T * K * 4, cudaMemcpyDeviceToDevice, s));
     }
     CU_TRY(h, cudaGetLastError());

@@ -250,16 +250,22 @@ permute_kernel(const void* __restrict__ x, int x_is_f32, int T, int H, int K, in
 // out[t,:] (+)= sum over the token's K assignments, ascending expert index, of
 // topk_w * y[slot,:].  gridDim.y blocks per token: one, or for a few tokens as many as
 // leave one vector to a thread, since the kernel is then a chain of load latencies.
+// SIDE: the caller's copies of the routing (topk_i_out, topk_w_out, either may be null) are stored
+// here, where the values are in shared memory.  Two device-to-device copies behind this kernel cost
+// 8 us of 141 (64 tokens, 32 experts, hidden 2880), the stores 1.  They come last: in front of the sum
+// they held its loads back (16384 tokens, combine 163 -> 184 us), so other calls run without them.
 // Expert-parallel peer mode: `wait_flags` points at this rank's G "results
 // delivered" flags; the block first waits (bounded) until every rank has stored
 // its result rows into y.  The grid then has at least one block even for T == 0:
 // the wait is also what keeps this rank from starting the next call while a peer
 // still reads what this call sent it.
+template <bool SIDE>
 __global__ void __launch_bounds__(256)
 combine_kernel(const float* __restrict__ y, int T, int H, int K, const int* __restrict__ topk_i,
                const float* __restrict__ topk_w, const int* __restrict__ slot_of,
-               float* __restrict__ out, int accumulate, const int* __restrict__ wait_flags, int G,
-               int seq, int* __restrict__ status) {
+               float* __restrict__ out, int accumulate, int* __restrict__ topk_i_out,
+               float* __restrict__ topk_w_out, const int* __restrict__ wait_flags, int G, int seq,
+               int* __restrict__ status) {
     // The routing is two kernels old and more: complete before this kernel starts, and read past
     // L1 because this kernel has not waited yet (ld_l2).  One warp reads it for the block: eight
     // warps asking L2 for the same words cost 8000 short rows 2 us of 31.
@@ -338,6 +344,13 @@ combine_kernel(const float* __restrict__ y, int T, int H, int K, const int* __re
             acc.x += p.x; acc.y += p.y; acc.z += p.z; acc.w += p.w;
         }
         o[v] = acc;
+    }
+    if (SIDE && blockIdx.y == 0 && (int)threadIdx.x < K) {
+        const int k = threadIdx.x;
+        if (topk_i_out)
+            topk_i_out[(size_t)t * K + k] = s_ex[k];
+        if (topk_w_out)
+            topk_w_out[(size_t)t * K + k] = s_wt[k];
     }
 }
 
