@@ -35,9 +35,8 @@
 // chunk (4352 B) stream at 2.6 TB/s over the whole GPU however deep the ring is,
 // copies of three chunks or more at 6.1 TB/s: a copy has a fixed cost.  (2) The
 // MMA-issuing warp needs ~25 cycles per tcgen05.mma at N = 32 (the tensor pipe's
-// own rate) but ~800 cycles per step around them -- one barrier test, one commit
-// and a little bookkeeping, each a round trip through a memory pipe that sixteen
-// decode warps keep busy -- and it is the only warp that can issue them.  Rings (of the
+// own rate) but ~400 cycles per step around them, in one thread and with nothing
+// else running -- and it is the only warp that can issue them.  Rings (of the
 // narrow form; Config holds the sizes of both):
 //   W ring   packed MXFP4 steps in shared memory (bulk copies; covers HBM latency)
 //   A ring   SA = 2 slots of 192 tensor-memory columns (decoded weights)
