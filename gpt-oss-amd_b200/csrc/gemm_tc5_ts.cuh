@@ -42,11 +42,18 @@
 //   A ring   SA = 2 slots of 192 tensor-memory columns (decoded weights)
 //   B ring   activation tiles in shared memory (one 3-d TMA box per step, no
 //            multicast), handed out in units of 24 KB: a step of an item with up to
-//            32 token rows takes one unit, with up to 64 rows two.  (Wide: three slots
-//            of 48 KB, one 2-d box per chunk)
+//            32 token rows takes one unit, with up to 64 rows two.  (Wide: four slots
+//            of 32 KB for a CTA's half of the rows, one 2-d box per chunk)
 // and NB barrier pairs indexed by the step number: full[i % NB] collects the
 // decode warps' arrivals and the TMA bytes of step i, empty[i % NB] is signalled
 // by tcgen05.commit when the MMAs of step i are done.
+//
+// An item of the wide form is a pair of weight tiles on a cluster of two CTAs: each decodes its own
+// tile into its own tensor memory and loads half the token rows, the leader issues
+// tcgen05.mma.cta_group::2 for both.  Its full[] barriers collect the decode warps of both CTAs.  The
+// activation tiles have barriers of their own: the leader's collects its copies and a forward by
+// warp 2 of the peer, which has seen the peer's copies complete there.
+// empty[] and tmem_full are multicast commits, tmem_empty collects both CTAs' epilogue warps.
 //
 // Warp roles:
 //   warp 0      W producer          warp 1   B producer (TMA)
@@ -85,17 +92,19 @@ constexpr int EPI_STAGE_BYTES = 2048;
 //   BN  most token rows of an item    CS  chunks of 64 K-columns per pipeline step
 //   SA  A slots (tensor memory)       SB  B slots (units of 32 rows where the item decides how
 //   WS  packed slots                      many it takes, BN rows where UNITS is false)
-// NB barrier pairs.  SA and WS are multiples of G, so the successive fills of a slot are handled
+// NB barrier pairs; PAIR: an item is two weight tiles on a CTA pair.  SA and WS are multiples of G, so the successive fills of a slot are handled
 // by one group in program order (an mbarrier parity wait cannot tell phase n from phase n-2).
-template <int BN_, int CS_, int SA_, int SB_, int WS_, int NB_, bool UNITS_>
+template <int BN_, int CS_, int SA_, int SB_, int WS_, int NB_, bool UNITS_, bool PAIR_>
 struct Config {
     static constexpr int BN = BN_, CS = CS_, SA = SA_, SB = SB_, WS = WS_, NB = NB_;
-    static constexpr bool UNITS = UNITS_;
-    static constexpr int B_SLOT_BYTES = CS * (UNITS ? 32 : BN) * 128;  // rows x 64 bf16 per chunk, SW128
+    static constexpr bool UNITS = UNITS_, PAIR = PAIR_;
+    static constexpr int ROW_GRANULE = PAIR ? 32 : 16;  // rows of an item: a multiple (each CTA of a pair loads half)
+    // rows x 64 bf16 per chunk, SW128
+    static constexpr int B_SLOT_BYTES = CS * (UNITS ? 32 : PAIR ? BN / 2 : BN) * 128;
     static constexpr int W_SLOT_BYTES = CS * CHUNK_BYTES;
     static constexpr int A_SLOT_COLS = CS * A_SUB_COLS;
     static constexpr int TMEM_A0 = SETS * BN;  // first tensor-memory column of the A slots
-    static constexpr int N_BARRIERS = 2 * WS + 2 * NB + 2 * SETS;
+    static constexpr int N_BARRIERS = 2 * WS + (PAIR ? 3 : 2) * NB + 2 * SETS;
     static constexpr int SMEM_BYTES = SB * B_SLOT_BYTES + WS * W_SLOT_BYTES + 4 * EPI_STAGE_BYTES + N_BARRIERS * 8 +
                                       (MAX_LOCAL_EXPERTS + 1) * 3 * 4 + 64 + 1024;
     static_assert(TMEM_A0 + SA * A_SLOT_COLS <= TMEM_COLS, "tensor memory");
@@ -106,24 +115,36 @@ struct Config {
 // Up to 64 rows per item: six chunks per step.  (Three chunks with four A slots, and three
 // decode warps per quarter instead of two, measured again on this form: 256 tokens, 32
 // experts 157 us per layer; 181 with three chunks, 167 with three warps.)
-using Narrow = Config<BN, STEP_CHUNKS, 2, 4, 4, 4, true>;
-// Up to 128 rows: a weight tile is decoded once for twice the rows.  Accumulators and B
-// tiles double, so a step has three chunks.  (Two chunks with four A slots: 777 tokens 285 us
-// instead of 258; four chunks with two B slots: 265.)
-using Wide = Config<BN_WIDE, 3, 2, 3, 4, 4, false>;
+using Narrow = Config<BN, STEP_CHUNKS, 2, 4, 4, 4, true, false>;
+// Up to 128 rows on CTA pairs: a weight tile is decoded once for twice the rows, and each CTA loads
+// half the token rows of an item, for at this height the activations are three times the packed
+// weights on the way from L2.  The halves leave room for four chunks per step.  Against one CTA per
+// item and three chunks (us per pass): 777 tokens, 32 experts 246 -> 238; 3001 tokens, 128 experts 962 -> 937;
+// 2048 x 768, 128 experts top-8, 1500 tokens 244 -> 236.
+using Wide = Config<BN_WIDE, 4, 2, 4, 4, 4, false, true>;
 
 // D[tmem] (+)= A[tmem] . B[smem desc]^T: A is 128 lanes x 8 columns (16 bf16 of K per lane).
 // The shared-memory descriptor comes as its two 32-bit halves: stepping through a tile
 // only changes the start-address field in the low half, one 32-bit add per MMA in the
 // issuing warp's chain instead of a 64-bit one.
+// PAIR: over a CTA pair, A is 128 lanes in each CTA's tensor memory, B half in each one's shared memory.
+template <bool PAIR>
 __device__ __forceinline__ void umma_ts_bf16(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_desc_lo,
                                              uint32_t b_desc_hi, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 bd;\n\t"
-        "mov.b64 bd, {%2, %3};\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %4, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "r"(b_desc_lo), "r"(b_desc_hi), "r"(idesc), "r"(accumulate) : "memory");
+    if (PAIR)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .b64 bd;\n\t"
+            "mov.b64 bd, {%2, %3};\n\t"
+            "setp.ne.b32 p, %5, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], bd, %4, p;\n\t}"
+            ::"r"(d_tmem), "r"(a_tmem), "r"(b_desc_lo), "r"(b_desc_hi), "r"(idesc), "r"(accumulate) : "memory");
+    else
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t.reg .b64 bd;\n\t"
+            "mov.b64 bd, {%2, %3};\n\t"
+            "setp.ne.b32 p, %5, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %4, p;\n\t}"
+            ::"r"(d_tmem), "r"(a_tmem), "r"(b_desc_lo), "r"(b_desc_hi), "r"(idesc), "r"(accumulate) : "memory");
 }
 // 32 lanes x 32 consecutive 32-bit columns: thread i of the warp writes lane (taddr.lane + i).
 __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t a[32]) {
@@ -142,7 +163,7 @@ __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.
 
 struct TileInfo {
     int e;        // local expert
-    int mt;       // 128-row weight tile
+    int mt;       // 128-row weight tile (PAIR: pair of them)
     int row0;     // first token row of the item
     int valid_n;  // token rows of the item (1..64, Wide 1..128)
     int n_mma;    // rows the MMA computes and the TMA box holds (a multiple of 16)
@@ -182,7 +203,7 @@ __device__ __forceinline__ TileInfo decode_tile(int tile, int m_tiles, const Til
     const int n0 = (r - ti.mt * ntl) * rows;
     ti.row0 = tt.off[lo] + n0;
     ti.valid_n = min(rows, cnt - n0);
-    ti.n_mma = (ti.valid_n + 15) & ~15;
+    ti.n_mma = (ti.valid_n + C::ROW_GRANULE - 1) & ~(C::ROW_GRANULE - 1);
     return ti;
 }
 
@@ -219,7 +240,14 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
     auto bar_tmem_full = [&](int b) { return bar0 + 8u * (uint32_t)(2 * C::WS + 2 * C::NB + b); };
     auto bar_tmem_empty = [&](int b) { return bar0 + 8u * (uint32_t)(2 * C::WS + 2 * C::NB + SETS + b); };
 
+    // activation tiles of a step: their own barriers in a pair, otherwise full[] counts them too
+    auto bar_b_full = [&](int s) {
+        return C::PAIR ? bar0 + 8u * (uint32_t)(2 * C::WS + 2 * C::NB + 2 * SETS + s) : bar_full(s);
+    };
+
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = C::PAIR ? cluster_ctarank() : 0;  // 0 = leader: issues the MMAs
+    const bool leader = rank == 0;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < C::WS; s++) {
@@ -227,18 +255,21 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
             mbar_init(bar_w_empty(s), GW);  // one elected arrival per warp of the decoding group
         }
         for (int s = 0; s < C::NB; s++) {
-            mbar_init(bar_full(s), GW + 1);  // the decode warps of a group + the TMA producer's expect_tx
-            mbar_init(bar_empty(s), 1);     // tcgen05.commit
+            // the decode warps of a group (in a pair: of both CTAs, at the leader), the producer's expect_tx
+            mbar_init(bar_full(s), C::PAIR ? 2 * GW : GW + 1);
+            if (C::PAIR)
+                mbar_init(bar_b_full(s), leader ? 2 : 1);  // expect_tx (at the leader: and the peer's forward)
+            mbar_init(bar_empty(s), 1);  // tcgen05.commit
         }
         for (int b = 0; b < SETS; b++) {
             mbar_init(bar_tmem_full(b), 1);
-            mbar_init(bar_tmem_empty(b), 4);  // one per epilogue warp
+            mbar_init(bar_tmem_empty(b), C::PAIR ? 8 : 4);  // one per epilogue warp (of both CTAs)
         }
         *abort_flag = 0;
         fence_barrier_init();
     }
     if (warp == MMA_WARP)
-        tmem_alloc(smem_u32(tmem_holder), TMEM_COLS);
+        C::PAIR ? tmem_alloc2(smem_u32(tmem_holder), TMEM_COLS) : tmem_alloc(smem_u32(tmem_holder), TMEM_COLS);
     // Everything above is this CTA's own set-up.  The gate/up launch waits here: its plan and
     // token rows come from the kernel before it.  Of what the down launch reads, only the
     // intermediate does (the plan is complete when it starts, pdl_trigger in common.cuh), so
@@ -255,6 +286,8 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
     }
     tc_fence_before();
     __syncthreads();
+    if (C::PAIR)
+        cluster_sync_all();  // the peer's barriers exist before anyone signals them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_holder;
     TileTables tt;
@@ -265,7 +298,19 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
     auto next_unit = [](int bu, int need) {  // SB is a power of two where an item takes several units
         return C::UNITS ? (bu + need) & (C::SB - 1) : (bu + 1 == C::SB ? 0 : bu + 1);
     };
-    const int total_tiles = tt.tile_start[E] * m_tiles;
+    const int m_units = C::PAIR ? (m_tiles + 1) / 2 : m_tiles;  // weight tiles, or pairs of them, per matrix
+    const int total_tiles = tt.tile_start[E] * m_units;
+    const int worker = C::PAIR ? (int)blockIdx.x >> 1 : (int)blockIdx.x;
+    const int n_workers = C::PAIR ? (int)gridDim.x >> 1 : (int)gridDim.x;
+    // This CTA's weight tile of an item.  The last pair of a matrix with an odd number of tiles has none
+    // for the peer: it decodes the leader's again (the MMA needs defined operands) and stores nothing.
+    auto my_tile = [&](int mt) { return C::PAIR ? min(2 * mt + (int)rank, m_tiles - 1) : mt; };
+    auto arrive_leader = [&](uint32_t bar) {
+        if (leader)
+            mbar_arrive(bar);
+        else
+            mbar_arrive_remote(bar, 0);
+    };
     const int n_steps = (k_stages + C::CS - 1) / C::CS;  // pipeline steps per work item; the last may hold fewer chunks
 
     if (warp == 0) {
@@ -276,10 +321,10 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
             bool ok = true;
             int wstep = 0;
             (void)wstep;
-            for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
-                const TileInfo ti = decode_tile<C>(tile, m_tiles, tt, E);
+            for (int tile = worker; ok && tile < total_tiles; tile += n_workers) {
+                const TileInfo ti = decode_tile<C>(tile, m_units, tt, E);
                 const uint8_t* wsrc = chunks + (size_t)ti.e * expert_stride +
-                                      (size_t)ti.mt * k_stages * CHUNK_BYTES;
+                                      (size_t)my_tile(ti.mt) * k_stages * CHUNK_BYTES;
                 for (int st = 0; st < n_steps; st++) {
                     ok = mbar_wait(bar_w_empty(s), ph ^ 1u, status, DS_TIMEOUT_EMPTY, abort_flag);
                     if (!ok)
@@ -331,10 +376,12 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                 if (!ok)
                     *abort_flag = 1;
             }
-            for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
-                const TileInfo ti = decode_tile<C>(tile, m_tiles, tt, E);
-                const int need = C::UNITS ? (ti.n_mma + 31) >> 5 : 1;  // units per step: 1 or 2
-                const uint32_t tile_bytes = (uint32_t)ti.n_mma * 128u;
+            for (int tile = worker; ok && tile < total_tiles; tile += n_workers) {
+                const TileInfo ti = decode_tile<C>(tile, m_units, tt, E);
+                const int rows = C::PAIR ? ti.n_mma >> 1 : ti.n_mma;  // that this CTA loads
+                const int row0 = ti.row0 + (int)rank * rows;
+                const int need = C::UNITS ? (rows + 31) >> 5 : 1;  // units per step: 1 or 2
+                const uint32_t tile_bytes = (uint32_t)rows * 128u;
                 for (int st = 0; st < n_steps; st++, i++) {
                     if (C::UNITS && need == 2 && (bu & 1))
                         bu = (bu + 1) & (C::SB - 1);
@@ -351,14 +398,14 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                     const uint32_t dst = smem_u32(b_ring + bu * C::B_SLOT_BYTES);
                     if (C::UNITS) {
                         // the whole box is delivered (chunks past the end of K arrive as zeros)
-                        mbar_expect_tx(bar_full(nb), (uint32_t)C::CS * tile_bytes);
-                        tma_load_3d(dst, &maps.box3[(ti.n_mma >> 4) - 1], bar_full(nb), 0, ti.row0, st * C::CS);
+                        mbar_expect_tx(bar_b_full(nb), (uint32_t)C::CS * tile_bytes);
+                        tma_load_3d(dst, &maps.box3[(rows >> 4) - 1], bar_b_full(nb), 0, row0, st * C::CS);
                     } else {
                         const int nch = min(C::CS, k_stages - st * C::CS);
-                        mbar_expect_tx(bar_full(nb), (uint32_t)nch * tile_bytes);
+                        mbar_expect_tx(bar_b_full(nb), (uint32_t)nch * tile_bytes);
                         for (int j = 0; j < nch; j++)
-                            tma_load_2d(dst + (uint32_t)j * tile_bytes, &maps.box[(ti.n_mma >> 4) - 1], bar_full(nb),
-                                        (st * C::CS + j) * KSTAGE, ti.row0);
+                            tma_load_2d(dst + (uint32_t)j * tile_bytes, &maps.box[(rows >> 4) - 1], bar_b_full(nb),
+                                        (st * C::CS + j) * KSTAGE, row0);
                     }
                     TRACE(i, 3);
                     bu = next_unit(bu, need);
@@ -384,13 +431,30 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
         // issue against this, us per layer, hidden 2880: 32 experts, 1 token with the norm 44.8 -> 43.7,
         // 16 tokens 124.1 -> 119.3, 64 tokens 133.5 -> 128.5, 256 tokens 140.7 -> 136; 128 experts,
         // 200 tokens 446 -> 428).
-        if (elect_one_sync()) {
+        auto commit = [](uint32_t bar) { C::PAIR ? umma2_commit_both(bar) : umma_commit(bar); };
+        if (C::PAIR && !leader) {
+            // the peer's activation tiles have landed: forwarded to the leader
+            if (elect_one_sync()) {
+                int nb = 0;
+                uint32_t ph = 0;
+                bool ok = true;
+                for (int tile = worker; ok && tile < total_tiles; tile += n_workers) {
+                    for (int st = 0; st < n_steps; st++) {
+                        ok = mbar_wait_hot(bar_b_full(nb), ph, status, DS_TIMEOUT_FULL_B, abort_flag);
+                        if (!ok)
+                            break;
+                        mbar_arrive_remote(bar_b_full(nb), 0);
+                        RING_ADVANCE(nb, ph, C::NB);
+                    }
+                }
+            }
+        } else if (elect_one_sync()) {
             int sa = 0, bu = 0, nb = 0;  // step i: A slot i % SA, barriers i % NB, B units as the producer hands them out
             uint32_t ph = 0;             // (i / NB) & 1
             bool ok = true;
             int it = 0;
-            for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++it) {
-                const TileInfo ti = decode_tile<C>(tile, m_tiles, tt, E);
+            for (int tile = worker; ok && tile < total_tiles; tile += n_workers, ++it) {
+                const TileInfo ti = decode_tile<C>(tile, m_units, tt, E);
                 const int set = it % SETS, round = it / SETS;
                 ok = mbar_wait(bar_tmem_empty(set), (uint32_t)(round & 1) ^ 1u, status, DS_TIMEOUT_TMEM_EMPTY,
                                abort_flag);
@@ -399,11 +463,13 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                 tc_fence_after();  // the epilogue's tcgen05.ld of this set came before
                 TRACE(it * n_steps, 12);
                 const uint32_t d_tmem = tmem_base + (uint32_t)(set * C::BN);
-                const uint32_t idesc = make_idesc(ti.n_mma);
-                const int need = C::UNITS ? (ti.n_mma + 31) >> 5 : 1;  // B units per step
-                const uint32_t sub_step = (uint32_t)ti.n_mma * 8u;  // one chunk's tile in descriptor units of 16 bytes
+                const uint32_t idesc = C::PAIR ? make_idesc2(ti.n_mma) : make_idesc(ti.n_mma);
+                const int rows = C::PAIR ? ti.n_mma >> 1 : ti.n_mma;  // token rows in this CTA's shared memory
+                const int need = C::UNITS ? (rows + 31) >> 5 : 1;     // B units per step
+                const uint32_t sub_step = (uint32_t)rows * 8u;  // one chunk's tile in descriptor units of 16 bytes
                 for (int st = 0; st < n_steps; st++) {
-                    ok = mbar_wait_hot(bar_full(nb), ph, status, DS_TIMEOUT_FULL_A, abort_flag);
+                    ok = !C::PAIR || mbar_wait_hot(bar_b_full(nb), ph, status, DS_TIMEOUT_FULL_B, abort_flag);
+                    ok = ok && mbar_wait_hot(bar_full(nb), ph, status, DS_TIMEOUT_FULL_A, abort_flag);
                     if (!ok)
                         break;
                     TRACE(it * n_steps + st, 4);
@@ -419,12 +485,12 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                         if (j < nch) {
 #pragma unroll
                             for (int kk = 0; kk < KSTAGE / 16; kk++)
-                                umma_ts_bf16(d_tmem, a_tmem + (uint32_t)(j * A_SUB_COLS + kk * 8),
+                                umma_ts_bf16<C::PAIR>(d_tmem, a_tmem + (uint32_t)(j * A_SUB_COLS + kk * 8),
                                              b_lo + (uint32_t)j * sub_step + (uint32_t)(kk * 2), b_hi, idesc,
                                              (st | j | kk) != 0 ? 1u : 0u);
                         }
                     }
-                    umma_commit(bar_empty(nb));  // frees both slots when these MMAs have read them
+                    commit(bar_empty(nb));  // frees both slots when these MMAs have read them
                     TRACE(it * n_steps + st, 5);
                     RING_ADVANCE(nb, ph, C::NB);
                     if (++sa == C::SA)
@@ -432,7 +498,7 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                     bu = next_unit(bu, need);
                 }
                 if (ok)
-                    umma_commit(bar_tmem_full(set));
+                    commit(bar_tmem_full(set));
             }
         }
         __syncwarp();
@@ -447,8 +513,7 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
         const int half = ((u >> 5) % GW) >> 2;  // 0: this warp takes chunks 0, 2, 4 of a step; 1: chunks 1, 3, 5
         const int r = (warp & 3) * 32 + lane;
         const uint32_t a_lane = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)C::TMEM_A0;
-        const int my_tiles = (int)blockIdx.x < total_tiles
-                                 ? (total_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+        const int my_tiles = worker < total_tiles ? (total_tiles - 1 - worker) / n_workers + 1 : 0;
         const int total_steps = my_tiles * n_steps;
         bool ok = true;
         for (int i = g; ok && i < total_steps; i += G) {
@@ -527,7 +592,7 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
             tc_fence_before();
             __syncwarp();
             if (lane == 0)
-                mbar_arrive(bar_full(nb));
+                arrive_leader(bar_full(nb));
             if ((u & (GW * 32 - 1)) == 0)
                 TRACE(i, 9);
         }
@@ -541,14 +606,14 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
         unsigned char* stage = epi_stage + (warp - EPI_WARP0) * EPI_STAGE_BYTES;
         bool ok = true;
         int it = 0;
-        for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++it) {
-            const TileInfo ti = decode_tile<C>(tile, m_tiles, tt, E);
+        for (int tile = worker; ok && tile < total_tiles; tile += n_workers, ++it) {
+            const TileInfo ti = decode_tile<C>(tile, m_units, tt, E);
             const int set = it % SETS, round = it / SETS;
             // Bias and 2^shift of this lane's weight row, cold in HBM: fetched while the MMAs of
             // the item run, so that the last item of a launch does not wait for them.
-            const int mt = ti.mt;
+            const int mt = C::PAIR ? 2 * ti.mt + (int)rank : ti.mt;
             const int m = mt * TILE_M + row;
-            const bool m_ok = MODE == 0 || m < out_rows_valid;  // 2I is a multiple of TILE_M: always in range
+            const bool m_ok = mt < m_tiles && (MODE == 0 || m < out_rows_valid);  // 2I is a multiple of TILE_M
             const float bm = m_ok ? __ldg(bias + (size_t)ti.e * bias_stride + m) : 0.f;
             const float rs = m_ok ? __ldg(rscale + (size_t)ti.e * bias_stride + m) : 1.f;
             ok = mbar_wait(bar_tmem_full(set), (uint32_t)(round & 1), status, DS_TIMEOUT_TMEM_FULL,
@@ -560,7 +625,9 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                 TRACE(it * n_steps, 10);
             tc_fence_after();
             const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(set * C::BN);
-            if (MODE == 0) {
+            if (mt >= m_tiles) {
+                // the missing half of the last pair
+            } else if (MODE == 0) {
                 // Lanes 2p / 2p+1 hold the gate / up row of feature pair p.  After one
                 // exchange the even lane finishes columns c0..c0+15 of that feature and
                 // the odd lane columns c0+16..c0+31; the warp's 32 token rows x 16
@@ -638,7 +705,7 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
             tc_fence_before();
             __syncwarp();
             if (lane == 0)
-                mbar_arrive(bar_tmem_empty(set));
+                arrive_leader(bar_tmem_empty(set));
             if (warp == EPI_WARP0 && lane == 0)
                 TRACE(it * n_steps, 11);
         }
@@ -649,9 +716,11 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
     // common exit: every role comes here, finished or aborted
     tc_fence_before();
     __syncthreads();
+    if (C::PAIR)
+        cluster_sync_all();  // nobody signals a CTA that has gone
     if (warp == MMA_WARP) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, TMEM_COLS);
+        C::PAIR ? tmem_dealloc2(tmem_base, TMEM_COLS) : tmem_dealloc(tmem_base, TMEM_COLS);
     }
     if (MODE == 1 && pio.ticket && threadIdx.x == 0) {
         // the last CTA to get here raises "results delivered" at every rank

@@ -94,6 +94,7 @@ struct moe_b200_handle_s {
 
     tc5::TensorMaps maps_x{}, maps_h{};  // TMA maps over the GEMM inputs
     int pair_grid = 0;       // CTAs of the pair GEMM (2 x resident clusters)
+    int ts_pair_grid = 0;    // the same of the pairs with weights in tensor memory
     int smem_attr_done = 0;  // bit set: shared-memory opt-in of a kernel family done on this device
 
     ep::State ep;
@@ -150,20 +151,38 @@ bool pdl_enabled() {
     return on;
 }
 
+// `cluster` CTAs per thread-block cluster (1: none).
 template <typename... KArgs, typename... Args>
-cudaError_t launch_kernel(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                          cudaStream_t st, Args&&... args) {
+cudaError_t launch_clusters(int cluster, bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                            cudaStream_t st, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster;
+        attr[n].val.clusterDim.y = 1;
+        attr[n].val.clusterDim.z = 1;
+        n++;
+    }
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n].val.programmaticStreamSerializationAllowed = 1;
+        n++;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch_kernel(bool pdl, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                          cudaStream_t st, Args&&... args) {
+    return launch_clusters(1, pdl, kernel, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
 template <typename T>
@@ -241,8 +260,12 @@ constexpr int FRONT_MAX_SMEM = 220 * 1024;
 // 128-row items / CTA pairs 258 / 305 and 277 / 320; 128 experts, 3001 tokens 1102 / 1183 and
 // 1054 / 1101; 2048 x 768, 128 experts top-8, 1500 tokens (11 and 16 times) 292 / 308 and
 // 268 / 297.
+// Those are figures of 128-row items with one CTA each.  On CTA pairs (128-row items / the large-batch
+// kernel): 32 experts, 1000 tokens (125 rows) 268 / 301, 1250 tokens (156 rows) 320 / 313; 128 experts, 4000
+// tokens (125 rows) 1008 / 1043, 4500 tokens (140 rows) 1130 / 1083.  Beyond 128 rows the average
+// expert needs two items.
 constexpr int SMALL_MAX_ROWS_PER_EXPERT = 56;
-constexpr int WIDE_MAX_ROWS_PER_EXPERT = 112;
+constexpr int WIDE_MAX_ROWS_PER_EXPERT = 128;
 
 // Token rows per routing block (16 x the router kernel's MT).  Measured (E = 128, route
 // stage in ms; block height, CTAs per cluster): 2048 tokens (16,1) 0.030, (32,1) 0.042,
@@ -455,6 +478,28 @@ cudaError_t launch_front(moe_b200_handle h, const LayerWeights& lw, const void* 
     return launch_front_nt<8>(h, lw, t, is_f32, rms_w, rms_w_is_f32, T, bn, score_out, pdl, st);
 }
 
+// CTAs of a persistent kernel that runs in clusters of two: it must not launch more clusters
+// than can be resident at once.
+moe_b200_status pair_grid_of(moe_b200_handle h, const void* kernel, int threads, size_t smem, int* grid) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * (h->n_sms / 2));
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n_clusters = 0;
+    CU_TRY(h, cudaOccupancyMaxActiveClusters(&n_clusters, kernel, &cfg));
+    if (n_clusters < 1)
+        return fail(h, MOE_B200_ERR_CUDA, "no CTA pair of the expert GEMM fits on this device");
+    *grid = 2 * std::min(n_clusters, h->n_sms / 2);
+    return MOE_B200_OK;
+}
+
 // Large batches on CTA pairs (gemm_tc5_pair.cuh): cluster launch, one cluster per SM pair.
 template <int MODE>
 moe_b200_status launch_pair_kernel(moe_b200_handle h, int grid, cudaStream_t st,
@@ -465,22 +510,10 @@ moe_b200_status launch_pair_kernel(moe_b200_handle h, int grid, cudaStream_t st,
                                    void* out, int out_ld, int out_valid, const int* row_dst,
                                    const peer::GemmPeerIO& pio) {
     namespace pr = tc5::pair;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(pr::N_THREADS);
-    cfg.dynamicSmemBytes = pr::SMEM_BYTES;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    CU_TRY(h, cudaLaunchKernelEx(&cfg, pr::expert_gemm_pair_kernel<MODE>, maps, chunks, stride, ks, m_tiles,
-                                 bias, rscale, bias_stride, g_off, g_cnt, g_tile_start, EL, out, out_ld,
-                                 out_valid,
-                                 row_dst, pio, h->cfg.swiglu_alpha, h->cfg.swiglu_limit, h->status));
+    CU_TRY(h, launch_clusters(2, false, pr::expert_gemm_pair_kernel<MODE>, dim3(grid), dim3(pr::N_THREADS),
+                              pr::SMEM_BYTES, st, maps, chunks, stride, ks, m_tiles, bias, rscale, bias_stride,
+                              g_off, g_cnt, g_tile_start, EL, out, out_ld, out_valid, row_dst, pio,
+                              h->cfg.swiglu_alpha, h->cfg.swiglu_limit, h->status));
     return MOE_B200_OK;
 }
 
@@ -495,23 +528,10 @@ moe_b200_status launch_pair(moe_b200_handle h, const LayerWeights& lw, const tc5
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, pr::SMEM_BYTES));
         CU_TRY(h, cudaFuncSetAttribute(pr::expert_gemm_pair_kernel<1>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, pr::SMEM_BYTES));
-        // clusters that can be resident at once: a persistent kernel must not launch more
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * (h->n_sms / 2));
-        cfg.blockDim = dim3(pr::N_THREADS);
-        cfg.dynamicSmemBytes = pr::SMEM_BYTES;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        int n_clusters = 0;
-        CU_TRY(h, cudaOccupancyMaxActiveClusters(&n_clusters, pr::expert_gemm_pair_kernel<0>, &cfg));
-        if (n_clusters < 1)
-            return fail(h, MOE_B200_ERR_CUDA, "no CTA pair of the expert GEMM fits on this device");
-        h->pair_grid = 2 * std::min(n_clusters, h->n_sms / 2);
+        const moe_b200_status sg = pair_grid_of(h, (const void*)pr::expert_gemm_pair_kernel<0>, pr::N_THREADS,
+                                                pr::SMEM_BYTES, &h->pair_grid);
+        if (sg)
+            return sg;
         h->smem_attr_done |= 4;
     }
     prof_mark(h, MOE_B200_STAGE_GEMM1, true, st);
@@ -545,17 +565,25 @@ moe_b200_status launch_ts(moe_b200_handle h, const LayerWeights& lw, const tc5::
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
         CU_TRY(h, cudaFuncSetAttribute(ts::expert_gemm_ts_kernel<1, C>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+        if (C::PAIR) {
+            const moe_b200_status sg = pair_grid_of(h, (const void*)ts::expert_gemm_ts_kernel<0, C>, ts::N_THREADS,
+                                                    C::SMEM_BYTES, &h->ts_pair_grid);
+            if (sg)
+                return sg;
+        }
         h->smem_attr_done |= ATTR;
     }
+    const int grid = C::PAIR ? h->ts_pair_grid : h->n_sms;
+    constexpr int CLUSTER = C::PAIR ? 2 : 1;
     prof_mark(h, MOE_B200_STAGE_GEMM1, true, st);
     const bool pdl = c.ep_size == 1 && pdl_enabled();
-    CU_TRY(h, launch_kernel(pdl, ts::expert_gemm_ts_kernel<0, C>, dim3(h->n_sms), dim3(ts::N_THREADS),
+    CU_TRY(h, launch_clusters(CLUSTER, pdl, ts::expert_gemm_ts_kernel<0, C>, dim3(grid), dim3(ts::N_THREADS),
                             C::SMEM_BYTES, st, maps_x, lw.w1, h->stride1, h->ks1, h->m_tiles1, lw.bias1,
                             lw.rscale1, 2 * I, g_off, g_cnt, g_tile_start, EL, (void*)h->hbuf, I, I,
                             (const int*)nullptr, pio, c.swiglu_alpha, c.swiglu_limit, h->status));
     prof_mark(h, MOE_B200_STAGE_GEMM1, false, st);
     prof_mark(h, MOE_B200_STAGE_GEMM2, true, st);
-    CU_TRY(h, launch_kernel(pdl, ts::expert_gemm_ts_kernel<1, C>, dim3(h->n_sms), dim3(ts::N_THREADS),
+    CU_TRY(h, launch_clusters(CLUSTER, pdl, ts::expert_gemm_ts_kernel<1, C>, dim3(grid), dim3(ts::N_THREADS),
                             C::SMEM_BYTES, st, h->maps_h, lw.w2, h->stride2, h->ks2, h->m_tiles2, lw.bias2,
                             lw.rscale2, H, g_off, g_cnt, g_tile_start, EL, (void*)yout, H, H, row_dst, pio,
                             c.swiglu_alpha, c.swiglu_limit, h->status));
