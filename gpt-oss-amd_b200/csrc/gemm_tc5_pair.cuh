@@ -275,6 +275,12 @@ expert_gemm_pair_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* 
                         nb = 0;
                 }
             }
+            // the commits of the last steps too must have arrived before this CTA exits (they are
+            // not ordered with that of tmem_full, which the epilogue has seen: gemm_tc5_ts.cuh)
+            for (int n = min(i, SB); ok && n > 0; n--) {
+                ok = mbar_wait(bar_empty(eb), phe, status, DS_TIMEOUT_EMPTY, abort_flag);
+                RING_ADVANCE(eb, phe, NB);
+            }
             if (!ok && i > 0) {
                 // after an abort: give the copies in flight 0.1 s to land before the CTA
                 // exits (their barriers also count decode arrivals that may never come,

@@ -413,6 +413,13 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
                         nb = 0;
                 }
             }
+            // The commits of the last steps too must have arrived before this CTA exits.  The
+            // epilogue sees only tmem_full complete, another commit, and nothing orders the
+            // arrivals of two: a late one would land in the barriers of the next kernel's CTA.
+            for (; ok && waited < i; waited++) {
+                ok = mbar_wait(bar_empty(waited % C::NB), (uint32_t)(waited / C::NB) & 1u, status, DS_TIMEOUT_EMPTY,
+                               abort_flag);
+            }
             if (!ok && i > 0) {
                 // after an abort: give the copies in flight 0.1 s to land before the CTA
                 // exits (their barriers also count decode arrivals that may never come,
