@@ -142,6 +142,24 @@ bool is_device_pointer(const void* p) {
     return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
 }
 
+// Whether a kernel on `device` may store 32-bit words at `p`: plain memory of that device, on a
+// word boundary.  Other memory is left to the copy engine, which reaches a GPU without peer access
+// and refuses what nobody can write.
+bool word_store_ok(const void* p, const cudaPointerAttributes& a, int device) {
+    return p && (reinterpret_cast<uintptr_t>(p) & 3u) == 0 && a.type == cudaMemoryTypeDevice && a.device == device;
+}
+
+bool word_store_ok(const void* p, int device) {
+    cudaPointerAttributes a;
+    if (!p)
+        return false;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return word_store_ok(p, a, device);
+}
+
 // Programmatic dependent launch (pdl_wait / pdl_trigger in common.cuh) for the kernels
 // of a small-batch single-GPU call: each may start its set-up while the kernel before
 // it drains.  MOE_B200_NO_PDL=1 in the environment switches it off (a debugging aid:
@@ -1207,14 +1225,14 @@ moe_b200_status forward_impl(moe_b200_handle h, int layer, const void* t, int t_
         // peer mode launches it for T == 0 as well: the wait inside is what orders this
         // rank's next call behind the peers' reads of this one
         prof_mark(h, MOE_B200_STAGE_COMBINE, true, s);
-        // the combine stores the routing for the caller too; a pointer that no int or float store may
-        // take gets a copy behind it
-        auto word_aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 3u) == 0; };
-        int* const ti_direct = word_aligned(topk_i_out) ? topk_i_out : nullptr;
-        float* const tw_direct = word_aligned(topk_w_out) ? topk_w_out : nullptr;
+        // the combine stores the routing for the caller too; memory that its stores may not touch
+        // gets a copy behind it
+        int* const ti_direct = word_store_ok(topk_i_out, c.device) ? topk_i_out : nullptr;
+        float* const tw_direct = word_store_ok(topk_w_out, c.device) ? topk_w_out : nullptr;
         const int combine_split = T <= 2 * h->n_sms && !peer_mode ? ceil_div(H / 4, 256) : 1;
         CU_TRY(h, launch_kernel(pdl, ti_direct || tw_direct ? combine_kernel<true> : combine_kernel<false>,
-                                dim3(T > 0 ? T : 1, combine_split), dim3(256), 0, s, y_for_combine, T, H, K, h->topk_i, h->topk_w, h->slot_of, out, accumulate, ti_direct, tw_direct,
+                                dim3(T > 0 ? T : 1, combine_split), dim3(256), 0, s, y_for_combine, T, H, K,
+                                h->topk_i, h->topk_w, h->slot_of, out, accumulate, ti_direct, tw_direct,
                                 combine_wait, c.ep_size, seq, h->status));
         prof_mark(h, MOE_B200_STAGE_COMBINE, false, s);
         h->last_launches++;
@@ -1695,6 +1713,16 @@ moe_b200_status moe_b200_unpack_resident(moe_b200_handle h, int layer, int local
 }
 
 }  // extern "C"
+
+#ifdef MOE_B200_TEST_AIDS
+// Not declared in the header: decisions of this file, for tests that have no GPU.
+extern "C" int moe_b200_test_word_store(int type, int owner, unsigned long long address, int device) {
+    cudaPointerAttributes a = {};
+    a.type = (cudaMemoryType)type;
+    a.device = owner;
+    return word_store_ok(reinterpret_cast<const void*>((uintptr_t)address), a, device);
+}
+#endif
 
 #if defined(MOE_B200_TEST_AIDS) && defined(TC5_TRACE)
 // Debug builds only (not declared in the header): reads the hand-off timestamps.

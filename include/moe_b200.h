@@ -151,7 +151,10 @@ moe_b200_status moe_b200_load_experts_file(moe_b200_handle h, const char* path, 
  *   router_score_out / topk_i_out / topk_w_out   optional device buffers
  *                [n_tokens, E] f32 / [n_tokens, K] i32 / [n_tokens, K] f32: the
  *                engine's observable side buffers (include/model.hpp:132-134);
- *                topk_w is after the softmax
+ *                topk_w is after the softmax.  Kernels of the handle's device
+ *                store router_score_out, and topk_* where it is memory of that
+ *                device on a 4-byte boundary; other topk_* memory (another GPU's,
+ *                pinned host, any alignment) gets a device-to-device copy
  * `t` and `out` must be 16-byte aligned (rows are moved 16 bytes at a time); a
  * pointer that is not is refused with MOE_B200_ERR_INVALID.
  * With ep_size > 1 every rank must call this for the same layer in the same
