@@ -91,13 +91,15 @@ constexpr int EPI_STAGE_BYTES = 2048;
 
 //   BN  most token rows of an item    CS  chunks of 64 K-columns per pipeline step
 //   SA  A slots (tensor memory)       SB  B slots (units of 32 rows where the item decides how
-//   WS  packed slots                      many it takes, BN rows where UNITS is false)
-// NB barrier pairs; PAIR: an item is two weight tiles on a CTA pair.  SA and WS are multiples of G, so the successive fills of a slot are handled
-// by one group in program order (an mbarrier parity wait cannot tell phase n from phase n-2).
+//   WS  packed slots                      many it takes, otherwise the rows that a CTA loads)
+// NB barrier pairs; PAIR: an item is two weight tiles on a CTA pair.  SA and WS are multiples of G,
+// so the successive fills of a slot are handled by one group in program order (an mbarrier parity
+// wait cannot tell phase n from phase n-2).
 template <int BN_, int CS_, int SA_, int SB_, int WS_, int NB_, bool UNITS_, bool PAIR_>
 struct Config {
     static constexpr int BN = BN_, CS = CS_, SA = SA_, SB = SB_, WS = WS_, NB = NB_;
     static constexpr bool UNITS = UNITS_, PAIR = PAIR_;
+    static constexpr int DECODE_UNROLL = UNITS || PAIR ? (CS + 1) / 2 : 1;  // chunks of a warp's share of a step
     static constexpr int ROW_GRANULE = PAIR ? 32 : 16;  // rows of an item: a multiple (each CTA of a pair loads half)
     // rows x 64 bf16 per chunk, SW128
     static constexpr int B_SLOT_BYTES = CS * (UNITS ? 32 : PAIR ? BN / 2 : BN) * 128;
@@ -116,12 +118,14 @@ struct Config {
 // decode warps per quarter instead of two, measured again on this form: 256 tokens, 32
 // experts 157 us per layer; 181 with three chunks, 167 with three warps.)
 using Narrow = Config<BN, STEP_CHUNKS, 2, 4, 4, 4, true, false>;
-// Up to 128 rows on CTA pairs: a weight tile is decoded once for twice the rows, and each CTA loads
-// half the token rows of an item, for at this height the activations are three times the packed
-// weights on the way from L2.  The halves leave room for four chunks per step.  Against one CTA per
-// item and three chunks (us per pass): 777 tokens, 32 experts 246 -> 238; 3001 tokens, 128 experts 962 -> 937;
-// 2048 x 768, 128 experts top-8, 1500 tokens 244 -> 236.
-using Wide = Config<BN_WIDE, 4, 2, 4, 4, 4, false, true>;
+// Up to 128 rows: a weight tile is decoded once for twice the rows.  Accumulators and B tiles double,
+// so a step has three chunks.  (Two chunks with four A slots: 777 tokens, 32 experts 285 us instead
+// of 258; four chunks with two B slots: 265.)
+using Wide = Config<BN_WIDE, 3, 2, 3, 4, 4, false, false>;
+// The same on CTA pairs: each CTA loads half the token rows of an item, for at this height the
+// activations are three times the packed weights on the way from L2.  The halves leave room for four
+// chunks per step.  Faster where there is enough to decode: wide_on_pairs in moe_b200.cu.
+using WidePair = Config<BN_WIDE, 4, 2, 4, 4, 4, false, true>;
 
 // D[tmem] (+)= A[tmem] . B[smem desc]^T: A is 128 lanes x 8 columns (16 bf16 of K per lane).
 // The shared-memory descriptor comes as its two 32-bit halves: stepping through a tile
@@ -540,8 +544,10 @@ expert_gemm_ts_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* __
             bool slot_free = false;
             // Unrolled: the packed bytes of a warp's next chunk are fetched and decoded while it stores
             // this one (us per pass, hidden 2880: 256 tokens x 24 layers, 32 experts 3575 -> 3467; 200
-            // tokens x 2 layers, 128 experts 917 -> 888).
-#pragma unroll
+            // tokens x 2 layers, 128 experts 917 -> 888).  Not in Wide, which runs where items are
+            // short (unrolled / not: 4096 x 256, 32 experts top-2, 1152 tokens 80.3 / 78.4; 2176 x 384,
+            // 101 experts top-2, 3636 tokens 166.5 / 163.2).
+#pragma unroll C::DECODE_UNROLL
             for (int jj = 0; jj < C::CS; jj += 2) {
                 const int j = jj + half;
                 if (j >= nch)

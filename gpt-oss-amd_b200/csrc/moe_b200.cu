@@ -268,22 +268,52 @@ constexpr int TC5_BN = 256;                   // token rows per tile of the larg
 // Shared memory of front_small_kernel: hidden sizes up to 8192 with 32 experts, 5120 with 128,
 // 2560 with 256; beyond, the separate kernels run.
 constexpr int FRONT_MAX_SMEM = 220 * 1024;
-// Rows per expert on average up to which the small-batch GEMM takes 64-row and 128-row
-// items.  Measured (hidden 2880, us per layer, 64-row items / 128-row items / CTA pairs):
-// 32 experts, 384 tokens (48 rows) 187 / 200 / -, 512 (64 rows) 234 / 220 / -, 777 (97 rows)
-// - / 255 / 303; 128 experts, 3001 tokens (94 rows) - / 990 / 1104, 4096 (128 rows) -
-// / 1329 / 1206.  The rule sees only the average, but skewed routing keeps the order (means of
-// runs in turn, busiest expert 4 / 7 times the average at 32 experts, 13 / 27 times at 128):
-// 32 experts, 464 tokens (58 rows), 64-row / 128-row items 210 / 211 and 237 / 232; 777 tokens,
-// 128-row items / CTA pairs 258 / 305 and 277 / 320; 128 experts, 3001 tokens 1102 / 1183 and
-// 1054 / 1101; 2048 x 768, 128 experts top-8, 1500 tokens (11 and 16 times) 292 / 308 and
-// 268 / 297.
-// Those are figures of 128-row items with one CTA each.  On CTA pairs (128-row items / the large-batch
-// kernel): 32 experts, 1000 tokens (125 rows) 268 / 301, 1250 tokens (156 rows) 320 / 313; 128 experts, 4000
-// tokens (125 rows) 1008 / 1043, 4500 tokens (140 rows) 1130 / 1083.  Beyond 128 rows the average
-// expert needs two items.
+// Rows per expert on average up to which a call takes 64-row and 128-row items (gemm_tc5_ts.cuh); beyond,
+// 256-row items (gemm_tc5_pair.cuh).  The rule sees only the average.  Measured, us per call, uniform
+// routing / busiest expert 4 and 6 times the average (32 experts) or 14 and 24 times (128):
+//   64-row against 128-row items, 2880 x 2880
+//     32 experts,  448 tokens (56 rows)   166, 195, 208   against   190, 206, 216
+//                  512 tokens (64 rows)   211, 197, 216             196, 208, 228
+//                  640 tokens (80 rows)   245, 236, 253             203, 235, 256
+//     128 experts, 2048 tokens (64 rows)  802, 817, 839             742, 852, 840
+//   128-row against 256-row items
+//     32 experts,  904 tokens (113 rows)  253, 268, 283   against   320, 329, 343
+//                  1024 tokens (128 rows) 292, 286, 312             324, 350, 372
+//                  1120 tokens (140 rows) 321, 310, 310             334, 370, 371
+//     128 experts, 3616 tokens (113 rows) 1029, 1105, 1170          1189, 1299, 1326
+//                  4096 tokens (128 rows) 1187, 1200, 1260          1225, 1336, 1422
+//                  4480 tokens (140 rows) 1298, 1256, 1345          1219, 1401, 1461
+//     2048 x 768, 128 experts top-8, 2048 tokens (128 rows)  292, 307, 322   against   320, 347, 365
+// 64-row items lose at 57 to 64 rows with uniform routing, later with skewed; past 128 rows the average
+// expert needs two 128-row items.
 constexpr int SMALL_MAX_ROWS_PER_EXPERT = 56;
 constexpr int WIDE_MAX_ROWS_PER_EXPERT = 128;
+
+// Whether 128-row items run on CTA pairs.  A pair decodes about 6 % faster, but its two launches cost
+// some 2 us more per call (as much as 1400 of the chunks below), and where a matrix has an odd number of
+// weight tiles the last pair decodes one for nothing.  `chunks`: 128 x 64 weight chunks of all local
+// experts, `idle` those of the missing tiles.  Measured from 57 to 128 rows per expert, one CTA per
+// item / pairs, us: 512 x 256, 16 experts (768 chunks), 776 tokens 32 / 35; 4096 x 256, 32 experts (12288),
+// 1152 tokens 78 / 82; 2816 x 448, 95 experts (43890, idle 4180), 2280 tokens 168 / 175; 1024 x 1408, 69
+// experts (36432), 1656 tokens 115 / 109; 2240 x 1920, 24 experts (38160), 776 tokens 98 / 95; 4096 x 2048, 16
+// experts (49152), 388 tokens 126 / 118; 2880 x 2880, 32 experts (97920, idle 2880), 776 tokens 225 / 219 and
+// skewed 258 / 251; 128 experts, 3104 tokens 918 / 905 and 1083 / 1058.  Over 47
+// shapes and 6 loads, pairs where this rule takes them are at most 2 % slower than one CTA per item.
+bool wide_on_pairs(int hidden, int intermediate, int n_local) {
+    const long long m1 = ceil_div(2 * intermediate, TILE_M), ks1 = hidden / KSTAGE;
+    const long long m2 = ceil_div(hidden, TILE_M), ks2 = intermediate / KSTAGE;
+    const long long chunks = n_local * (m1 * ks1 + m2 * ks2);
+    const long long idle = n_local * ((m1 & 1) * ks1 + (m2 & 1) * ks2);
+    return 6 * chunks > 100 * (idle + 1400);
+}
+
+// Rows per item for `rows` rows spread over the local experts.
+int item_rows(int rows, int n_local) {
+    const int per_expert = rows / (n_local > 0 ? n_local : 1);
+    if (per_expert <= SMALL_MAX_ROWS_PER_EXPERT)
+        return tc5::ts::BN;
+    return per_expert <= WIDE_MAX_ROWS_PER_EXPERT ? tc5::ts::BN_WIDE : TC5_BN;
+}
 
 // Token rows per routing block (16 x the router kernel's MT).  Measured (E = 128, route
 // stage in ms; block height, CTAs per cluster): 2048 tokens (16,1) 0.030, (32,1) 0.042,
@@ -644,14 +674,13 @@ moe_b200_status launch_gemms(moe_b200_handle h, const LayerWeights& lw, const ui
     }
 #endif
     (void)rows_upper;
-    (void)H;
-    (void)I;
-    (void)EL;
     (void)xin;
     if (bn == tc5::ts::BN)
         return launch_ts<tc5::ts::Narrow, 32>(h, lw, maps_x, g_off, g_cnt, g_tile_start, yout, row_dst, pio, st);
-    if (bn == tc5::ts::BN_WIDE)
-        return launch_ts<tc5::ts::Wide, 128>(h, lw, maps_x, g_off, g_cnt, g_tile_start, yout, row_dst, pio, st);
+    if (bn == tc5::ts::BN_WIDE) {
+        const auto launch = wide_on_pairs(H, I, EL) ? launch_ts<tc5::ts::WidePair, 256> : launch_ts<tc5::ts::Wide, 128>;
+        return launch(h, lw, maps_x, g_off, g_cnt, g_tile_start, yout, row_dst, pio, st);
+    }
     if (bn == TC5_BN)
         return launch_pair(h, lw, maps_x, g_off, g_cnt, g_tile_start, yout, row_dst, pio, st);
     return fail(h, MOE_B200_ERR_INVALID, "tile tables were built for another tile height");
@@ -666,19 +695,16 @@ int permute_split(moe_b200_handle h, int nblk, int n_assign) {
 
 // Token rows per GEMM tile for a call that has `rows` rows spread over the local
 // experts; the tile tables are built for it and it selects the kernel: few rows per
-// expert (bound by streaming the weights) -> the single-CTA kernel with the decoded
-// weights in tensor memory, 64 token rows per tile; a medium number -> the same kernel
-// with 128 token rows per tile; otherwise CTA pairs and 256 token rows per tile.  Any
-// choice is correct for any distribution of rows.
+// expert (bound by streaming the weights) or a medium number -> the kernel with the
+// decoded weights in tensor memory, 64 or 128 token rows per tile; otherwise the
+// large-batch kernel and 256 token rows per tile.  Any choice is correct for any
+// distribution of rows.
 int pick_bn(moe_b200_handle h, int rows) {
 #ifdef MOE_B200_TEST_AIDS
     if (h->cfg.gemm_impl == MOE_B200_GEMM_MMA_SYNC)
         return V0_BN;
 #endif
-    const int per_expert = rows / (h->n_local > 0 ? h->n_local : 1);
-    if (per_expert <= SMALL_MAX_ROWS_PER_EXPERT)
-        return tc5::ts::BN;
-    return per_expert <= WIDE_MAX_ROWS_PER_EXPERT ? tc5::ts::BN_WIDE : TC5_BN;
+    return item_rows(rows, h->n_local);
 }
 
 moe_b200_status check_shard(moe_b200_handle h, int first_expert, int n) {
@@ -1721,6 +1747,12 @@ extern "C" int moe_b200_test_word_store(int type, int owner, unsigned long long 
     a.type = (cudaMemoryType)type;
     a.device = owner;
     return word_store_ok(reinterpret_cast<const void*>((uintptr_t)address), a, device);
+}
+// Token rows of an item, and the CTAs that work on one.
+extern "C" int moe_b200_test_gemm_form(int hidden, int intermediate, int n_local, int rows, int* ctas) {
+    const int bn = item_rows(rows, n_local);
+    *ctas = bn == TC5_BN || (bn == moe::tc5::ts::BN_WIDE && wide_on_pairs(hidden, intermediate, n_local)) ? 2 : 1;
+    return bn;
 }
 #endif
 
