@@ -7,11 +7,13 @@ Every comparison returns -- and the tests print -- both the RAW max-abs error
 and the one left after removing the effect of identified one-ulp bf16 flips of
 the intermediate h; the raw figure has its own asserted ceiling.
 """
+import ctypes
+
 import numpy as np
 import torch
 
 import gpt_oss_amd_b200 as pkg
-from gpt_oss_amd_b200 import synth
+from gpt_oss_amd_b200 import capi, synth
 from oracle import oracle, parity
 from oracle.parity import tie_mask  # noqa: F401  (re-exported for the tests)
 
@@ -59,6 +61,15 @@ def compare_sampled(res, lw_or_loader, x_bits, w_router_bits, b_router, top_k, l
     m = parity.compare_sampled(res, x_bits, w_router_bits, b_router, loader, top_k, group=group)
     assert m["ok"], f"{label}: {m['why']}"
     return m
+
+
+def gemm_form(hidden, intermediate, n_local, rows):
+    """(token rows of an item, CTAs that work on one) of the expert GEMM that a call with `rows` rows over
+    `n_local` local experts takes."""
+    f = capi.lib(test_aids=True).moe_b200_test_gemm_form
+    f.argtypes = [ctypes.c_int] * 4 + [ctypes.POINTER(ctypes.c_int)]
+    ctas = ctypes.c_int()
+    return f(hidden, intermediate, n_local, rows, ctypes.byref(ctas)), ctas.value
 
 
 def run_gpu(shape, lw, x_bits, gemm_impl, dtype="bf16", max_tokens=None, accumulate_into=None,

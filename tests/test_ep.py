@@ -21,7 +21,7 @@ import torch.multiprocessing as mp
 import ep_workers
 import gpt_oss_amd_b200 as pkg
 from gpt_oss_amd_b200 import capi, synth
-from parity_util import compare, oracle_case, run_gpu
+from parity_util import compare, gemm_form, oracle_case, run_gpu
 
 
 def _free_port():
@@ -95,18 +95,23 @@ def test_expert_parallel_on_gpus(impl, mode):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("T,item_rows", [
+    (8192, 256),  # 256 rows per expert: the large-batch GEMM
+    (3200, 128),  # 100 rows: 128-row items on CTA pairs
+])
 @pytest.mark.parametrize("mode", ["nccl", "peer"])
-def test_expert_parallel_full_width_pair_kernel(mode):
-    """gpt-oss-120b-shaped layer (E = 128, H = I = 2880), 4096 tokens over all the GPUs
-    of the box: 128 rows per expert, i.e. the CTA-pair GEMM under expert parallelism.
-    Every rank checks eight of its own tokens against the CPU oracle."""
+def test_expert_parallel_full_width_pair_kernel(mode, T, item_rows):
+    """gpt-oss-120b-shaped layer (E = 128, H = I = 2880) over all the GPUs of the box: the
+    kernels that work on CTA pairs under expert parallelism.  Every rank checks eight of its
+    own tokens against the CPU oracle."""
     import json
 
     world = min(torch.cuda.device_count(), 8)
     if world < 2:
         pytest.skip("needs at least 2 GPUs")
-    T, seed = 4096, 0
+    seed = 0
     shape_kw = dict(hidden=2880, intermediate=2880, n_experts=128, top_k=4)
+    assert gemm_form(2880, 2880, 128 // world, T // world * 4) == (item_rows, 2)
     with tempfile.TemporaryDirectory() as d:
         mp.spawn(ep_workers.gpu_worker,
                  args=(world, _free_port(), shape_kw, T, seed, d, capi.GEMM_TCGEN05, mode, 8),

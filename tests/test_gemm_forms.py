@@ -1,6 +1,5 @@
 """Which form of the expert GEMM a call takes, and the two forms of its 128-row items, one CTA each
 or a CTA pair, on both sides of the line between them."""
-import ctypes
 import statistics
 
 import numpy as np
@@ -8,15 +7,7 @@ import pytest
 
 import gpt_oss_amd_b200 as pkg
 from gpt_oss_amd_b200 import capi, synth
-from parity_util import compare_sampled, run_gpu
-
-
-def form(hidden, intermediate, n_local, rows):
-    """(token rows of an item, CTAs that work on one)."""
-    f = capi.lib(test_aids=True).moe_b200_test_gemm_form
-    f.argtypes = [ctypes.c_int] * 4 + [ctypes.POINTER(ctypes.c_int)]
-    ctas = ctypes.c_int()
-    return f(hidden, intermediate, n_local, rows, ctypes.byref(ctas)), ctas.value
+from parity_util import compare_sampled, gemm_form, run_gpu
 
 
 @pytest.mark.parametrize("hidden,intermediate,n_local,ctas", [
@@ -28,9 +19,9 @@ def form(hidden, intermediate, n_local, rows):
 ])
 def test_form_of_128_row_items(hidden, intermediate, n_local, ctas):
     for rows in (57, 128):
-        assert form(hidden, intermediate, n_local, rows * n_local) == (128, ctas)
-    assert form(hidden, intermediate, n_local, 57 * n_local - 1) == (64, 1)
-    assert form(hidden, intermediate, n_local, 129 * n_local) == (256, 2)
+        assert gemm_form(hidden, intermediate, n_local, rows * n_local) == (128, ctas)
+    assert gemm_form(hidden, intermediate, n_local, 57 * n_local - 1) == (64, 1)
+    assert gemm_form(hidden, intermediate, n_local, 129 * n_local) == (256, 2)
 
 
 @pytest.mark.gpu
@@ -47,7 +38,7 @@ def test_128_row_items_in_both_forms(ctas, H, I, E, K, avg, few):
     of test_tcgen05_equals_mma_sync_at_prefill_size), a sample against the oracle.  `few`: hardly any
     rows for the last expert, so that boxes of its item lie past the last row of the buffer."""
     T = -(-avg * E // K)
-    assert form(H, I, E, T * K) == ((128, ctas) if avg <= 128 else (256, 2))
+    assert gemm_form(H, I, E, T * K) == ((128, ctas) if avg <= 128 else (256, 2))
     shape = pkg.MoEShape(hidden=H, intermediate=I, n_experts=E, top_k=K)
     lw = synth.make_layer(shape, seed=H + avg)
     if few:  # logits are N(0, 0.0004 H) over the experts: about six tokens choose the last one

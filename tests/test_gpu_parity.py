@@ -13,7 +13,7 @@ import torch
 import gpt_oss_amd_b200 as pkg
 from gpt_oss_amd_b200 import capi, synth
 from oracle import oracle
-from parity_util import compare, compare_sampled, oracle_case, run_gpu
+from parity_util import compare, compare_sampled, gemm_form, oracle_case, run_gpu
 
 pytestmark = pytest.mark.gpu
 
@@ -153,7 +153,8 @@ CASES = [
     (128, 64, 32, 4, 2500),   # above the small-batch routing threshold
     (128, 64, 128, 4, 2100),
     (320, 192, 4, 2, 700),    # large-batch GEMM kernel with partial weight tiles
-    (128, 64, 128, 4, 4000),  # large-batch (CTA-pair) GEMM kernel with 128 experts, 125 rows each
+    (128, 64, 128, 4, 4000),  # 128-row items with 128 experts, 125 rows each
+    (128, 64, 128, 4, 4600),  # large-batch GEMM kernel with 128 experts, 143 rows each
     (192, 128, 128, 4, 9000), # the same above 256 rows per expert: several token tiles per expert
     (128, 64, 64, 4, 9600),   # 64-token routing blocks (above 9472 tokens)
 ]
@@ -433,21 +434,30 @@ def test_forward_host_matches_device_path():
         assert torch.equal(out, dev)
 
 
-def test_forward_host_chunked_equals_device_path():
+@pytest.mark.parametrize("H,I,E,T,chunk,ctas", [
+    (128, 64, 8, 5000, 2560, None),        # two chunks, the large-batch GEMM in both calls
+    (128, 64, 128, 8192, 4096, 1),         # chunks of 128 rows per expert take 128-row items
+    (1024, 1024, 128, 8192, 4096, 2),      # the same on CTA pairs
+])
+def test_forward_host_chunked_equals_device_path(H, I, E, T, chunk, ctas):
     """Large batches go through the host-buffer entry point in token chunks whose
-    copies overlap the compute: same bits as one call on device buffers."""
-    shape = pkg.MoEShape(hidden=128, intermediate=64, n_experts=8, top_k=4)
+    copies overlap the compute: same bits as one call on device buffers, also where
+    the chunks are small enough for another form of the GEMM."""
+    shape = pkg.MoEShape(hidden=H, intermediate=I, n_experts=E, top_k=4)
+    assert gemm_form(H, I, E, T * 4) == (256, 2)
+    assert gemm_form(H, I, E, chunk * 4) == ((128, ctas) if ctas else (256, 2))
     lw = synth.make_layer(shape, seed=4)
-    T = 5000  # two chunks of 2560 tokens
-    x_bits = synth.make_tokens(T, 128, seed=4)
+    x_bits = synth.make_tokens(T, H, seed=4)
     with pkg.MoEEngine(shape, max_tokens=T) as eng:
         eng.load_layer(0, lw)
         t = torch.from_numpy(x_bits.view(np.int16)).view(torch.bfloat16)
         dev, _, ti, tw = eng.forward(0, t.cuda(), side=True)
         dev, ti, tw = dev.cpu(), ti.cpu(), tw.cpu()
-        out = torch.empty(T, 128, dtype=torch.float32).pin_memory()
-        eng.forward_host(0, t.pin_memory(), out)
-        assert torch.equal(out, dev)
+        out = torch.empty(T, H, dtype=torch.float32).pin_memory()
+        ti_host = torch.empty(T, 4, dtype=torch.int32).pin_memory()
+        tw_host = torch.empty(T, 4, dtype=torch.float32).pin_memory()
+        eng.forward_host(0, t.pin_memory(), out, ti_host, tw_host)
+        assert torch.equal(out, dev) and torch.equal(ti_host, ti) and torch.equal(tw_host, tw)
         assert eng.device_status() == 0
 
 

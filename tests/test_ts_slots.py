@@ -1,7 +1,7 @@
 """GPU parity of the GEMM with decoded weights in tensor memory where its rings are cut: K of one
-chunk (64 columns), one less and one more than a step holds, an odd number of weight tiles (a CTA
-pair without a second one), and items of one row.  The oracle and its tolerances are those of
-test_gpu_parity.py."""
+chunk (64 columns), one less and one more than a step holds, and items of one row; 64-row items and
+128-row items with one CTA each (on CTA pairs: test_gemm_forms.py).  The oracle and its tolerances are
+those of test_gpu_parity.py."""
 import pytest
 
 import gpt_oss_amd_b200 as pkg

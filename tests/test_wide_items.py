@@ -1,12 +1,13 @@
-"""GPU parity of the 128-row variant of the small-batch GEMM, at the sizes where its dispatch
-changes or a tile is cut.  The oracle and its tolerances are those of test_gpu_parity.py."""
+"""GPU parity of the 128-row items of the GEMM with decoded weights in tensor memory where a tile is
+cut or a ring comes round (test_gemm_forms.py: where its dispatch changes).  The oracle and its
+tolerances are those of test_gpu_parity.py."""
 import numpy as np
 import pytest
 import torch
 
 import gpt_oss_amd_b200 as pkg
 from gpt_oss_amd_b200 import capi, synth
-from parity_util import compare, compare_sampled, oracle_case, run_gpu
+from parity_util import compare, compare_sampled, gemm_form, oracle_case, run_gpu
 
 pytestmark = pytest.mark.gpu
 
@@ -30,8 +31,8 @@ def test_wide_items(H, I, E, K, T, skew):
 
 
 @pytest.mark.parametrize("H,I,E,K,T", [
-    (2880, 2880, 32, 4, 777),   # 15 steps per item
-    (1088, 832, 64, 4, 1600),   # 6 and 5 steps, the last one cut in both launches
+    (2880, 2880, 32, 4, 777),   # on CTA pairs: 12 steps per item
+    (1088, 832, 64, 4, 1600),   # one CTA per item: 6 and 5 steps, the last one cut in both launches
 ])
 @pytest.mark.parametrize("skew", [False, True])
 def test_wide_items_reuse_their_rings(H, I, E, K, T, skew):
@@ -46,9 +47,11 @@ def test_wide_items_reuse_their_rings(H, I, E, K, T, skew):
     res = run_gpu(shape, lw, x_bits, capi.GEMM_TCGEN05)  # asserts the status word
     items = sum(-(-c // 128) for c in res["counts"])
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    assert 57 * E <= sum(res["counts"]) < 113 * E  # the rule that picks this form
+    rows, ctas = gemm_form(H, I, E, sum(res["counts"]))
+    assert rows == 128
     for m_tiles, k in ((-(-2 * I // 128), H), (-(-H // 128), I)):
-        assert items * m_tiles >= 3 * sms and -(-k // 64 // 3) > 4
+        assert items * -(-m_tiles // ctas) >= 3 * (sms // ctas)  # three items and more to a CTA or pair
+        assert -(-k // 64 // (2 + ctas)) > 4  # steps of three or four chunks: more than the rings hold
     if skew:
         assert max(res["counts"]) > 256  # more than two items of one expert
     ref = run_gpu(shape, lw, x_bits, capi.GEMM_MMA_SYNC)
