@@ -312,8 +312,8 @@ expert_gemm_pair_kernel(const __grid_constant__ TensorMaps maps, const uint8_t* 
             // One thread runs the loop: each instruction between two steps delays the next MMAs, and votes,
             // elections and reconvergence of a whole warp were most of them (a whole warp, with the barrier
             // of the next step tested ahead, against this; us per layer, hidden 2880: 32 experts, 1000 tokens
-            // 306 -> 299, 2048 tokens 448 -> 441, 8192 skewed 1325 -> 1317; 128 experts, 4500 tokens
-            // 1092 -> 1085).
+            // 306 -> 299, 2048 tokens 448 -> 441; 128 experts, 4500 tokens 1092 -> 1085; from 8192 tokens on
+            // within the spread of the runs).
             int it = 0;
             for (int tile = pair_id; ok && tile < total_tiles; tile += n_pairs, ++it) {
                 const TileInfo ti = decode_tile(tile, m_pairs, tt, E);

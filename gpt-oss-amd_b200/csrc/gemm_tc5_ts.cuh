@@ -1,5 +1,5 @@
-// Grouped expert GEMMs for SMALL batches (few token rows per expert), tcgen05,
-// decoded weights in TENSOR MEMORY.
+// Grouped expert GEMMs for SMALL and MEDIUM batches (up to 128 token rows per expert on
+// average), tcgen05, decoded weights in TENSOR MEMORY.
 //
 //   MODE 0: h[rows, I]  = SwiGLU(x[rows, H] . W1_e^T + b1_e)      (bf16 out)
 //           moe_mlp1_swiglu, src/hip/moe.hip:9-258
@@ -26,30 +26,30 @@
 // chunk issue in ~100 cycles), shared memory carries only the packed bytes and the small
 // activation tile.
 //
-// One persistent CTA per SM walks work items (expert, 128-row weight tile, tile
-// of up to 64 token rows, or 128 in the wide variant: medium batches, where 64-row items
-// would decode most weights twice and CTA pairs run half-empty tiles; figures at Narrow and
-// Wide below).  A pipeline STEP of the narrow form covers CS = 6 chunks of 64 K-columns
+// Persistent CTAs, one per SM, walk work items.  Three forms (Narrow, Wide, WidePair below):
+// an item is (expert, 128-row weight tile, tile of up to 64 token rows), the same with up to
+// 128 (medium batches, where 64-row items would decode most weights twice and the 256-row
+// items of gemm_tc5_pair.cuh run half-empty), or that for two weight tiles on a CTA pair.
+// A pipeline STEP of the narrow form covers CS = 6 chunks of 64 K-columns
 // (384 columns, 26 KB of packed weights: one bulk copy, the chunks of a weight
 // tile are contiguous).  Two measurements set that size.  (1) Bulk copies of one
 // chunk (4352 B) stream at 2.6 TB/s over the whole GPU however deep the ring is,
 // copies of three chunks or more at 6.1 TB/s: a copy has a fixed cost.  (2) The
-// MMA-issuing warp needs ~25 cycles per tcgen05.mma at N = 32 (the tensor pipe's
-// own rate) but ~400 cycles per step around them, in one thread and with nothing
-// else running -- and it is the only warp that can issue them.  Rings (of the
-// narrow form; Config holds the sizes of both):
+// MMA-issuing thread needs 22 cycles per tcgen05.mma beside the decode warps and some 400
+// cycles per step around them (a loop of nothing but MMAs at N = 16: 8 and 300) -- and it
+// is the only one that can issue them.  Rings (of the narrow form; Config holds all sizes):
 //   W ring   packed MXFP4 steps in shared memory (bulk copies; covers HBM latency)
 //   A ring   SA = 2 slots of 192 tensor-memory columns (decoded weights)
 //   B ring   activation tiles in shared memory (one 3-d TMA box per step, no
 //            multicast), handed out in units of 24 KB: a step of an item with up to
-//            32 token rows takes one unit, with up to 64 rows two.  (Wide: four slots
-//            of 32 KB for a CTA's half of the rows, one 2-d box per chunk)
+//            32 token rows takes one unit, with up to 64 rows two.  (Wide, WidePair:
+//            slots of 48 KB and, for a CTA's half of the rows, 32 KB; a 2-d box per chunk)
 // and NB barrier pairs indexed by the step number: full[i % NB] collects the
 // decode warps' arrivals and the TMA bytes of step i, empty[i % NB] is signalled
 // by tcgen05.commit when the MMAs of step i are done.
 //
-// An item of the wide form is a pair of weight tiles on a cluster of two CTAs: each decodes its own
-// tile into its own tensor memory and loads half the token rows, the leader issues
+// On a CTA pair each CTA decodes its own tile into its own tensor memory and loads half the token
+// rows, the leader issues
 // tcgen05.mma.cta_group::2 for both.  Its full[] barriers collect the decode warps of both CTAs.  The
 // activation tiles have barriers of their own: the leader's collects its copies and a forward by
 // warp 2 of the peer, which has seen the peer's copies complete there.
@@ -76,7 +76,7 @@ namespace tc5 {
 namespace ts {
 
 constexpr int BN = 64;                       // most token rows per work item (UMMA N)
-constexpr int BN_WIDE = 128;                 // the same of the wide variant
+constexpr int BN_WIDE = 128;                 // the same of the wide variants
 constexpr int A_SUB_COLS = KSTAGE / 2;       // one decoded chunk in tensor memory: 128 lanes x 32 columns of bf16x2
 constexpr int MMA_WARP = 2;
 constexpr int DEQ_WARP0 = 3;
@@ -169,8 +169,8 @@ struct TileInfo {
     int e;        // local expert
     int mt;       // 128-row weight tile (PAIR: pair of them)
     int row0;     // first token row of the item
-    int valid_n;  // token rows of the item (1..64, Wide 1..128)
-    int n_mma;    // rows the MMA computes and the TMA box holds (a multiple of 16)
+    int valid_n;  // token rows of the item (1..BN)
+    int n_mma;    // rows the MMA computes and the TMA boxes hold (a multiple of ROW_GRANULE)
 };
 
 struct TileTables {

@@ -93,8 +93,8 @@ struct moe_b200_handle_s {
     int* stage_shift = nullptr;  // exponent shift of every row of the matrix being re-tiled
 
     tc5::TensorMaps maps_x{}, maps_h{};  // TMA maps over the GEMM inputs
-    int pair_grid = 0;       // CTAs of the pair GEMM (2 x resident clusters)
-    int ts_pair_grid = 0;    // the same of the pairs with weights in tensor memory
+    int pair_grid = 0;       // CTAs of the large-batch GEMM (2 x resident clusters)
+    int ts_pair_grid = 0;    // the same of the 128-row items on CTA pairs
     int smem_attr_done = 0;  // bit set: shared-memory opt-in of a kernel family done on this device
 
     ep::State ep;
@@ -548,7 +548,7 @@ moe_b200_status pair_grid_of(moe_b200_handle h, const void* kernel, int threads,
     return MOE_B200_OK;
 }
 
-// Large batches on CTA pairs (gemm_tc5_pair.cuh): cluster launch, one cluster per SM pair.
+// Large batches, 256-row items on CTA pairs (gemm_tc5_pair.cuh): cluster launch, one cluster per SM pair.
 template <int MODE>
 moe_b200_status launch_pair_kernel(moe_b200_handle h, int grid, cudaStream_t st,
                                    const tc5::TensorMaps& maps, const uint8_t* chunks, size_t stride,
@@ -600,7 +600,7 @@ moe_b200_status launch_pair(moe_b200_handle h, const LayerWeights& lw, const tc5
     return MOE_B200_OK;
 }
 
-// Small batches, decoded weights in tensor memory (gemm_tc5_ts.cuh).  ATTR: bit of smem_attr_done.
+// Small and medium batches, decoded weights in tensor memory (gemm_tc5_ts.cuh).  ATTR: bit of smem_attr_done.
 template <class C, int ATTR>
 moe_b200_status launch_ts(moe_b200_handle h, const LayerWeights& lw, const tc5::TensorMaps& maps_x,
                           const int* g_off, const int* g_cnt, const int* g_tile_start, float* yout,
@@ -1309,9 +1309,11 @@ moe_b200_status moe_b200_forward_host(moe_b200_handle h, int layer, const void* 
     // The block is independent per token, and a row's result does not depend on which
     // rows share its tile (the K loop has a fixed order), so a large batch is cut into
     // token chunks whose host->device copy, compute and device->host copy overlap on
-    // three streams: the copies (PCIe, the fp32 result above all) take longer than the
-    // compute.  A chunk keeps >= 128 rows per expert (measured at 16384 tokens, 128 experts:
-    // 5.97-6.38 ms per step with four chunks, 6.42-7.43 with two).
+    // three streams: the copies (PCIe, the fp32 result above all) take about as long as
+    // the compute.  A chunk keeps >= 128 rows per expert (us per call, 128 experts, as here / with two
+    // chunks at most: 12288 tokens 4408 / 4501, 15000 tokens 5040 / 5524, 16384 tokens 5436 / 5998).  At
+    // exactly 128 -- batches that are multiples of it -- the chunks take 128-row items: 8192, 12288 and
+    // 16384 tokens gained 5 to 6 % from that, 10000 and 15000 tokens 1 to 2 %.
     // Not with expert parallelism: every call is collective there and the ranks' token
     // counts differ.
     int chunk = n_tokens;

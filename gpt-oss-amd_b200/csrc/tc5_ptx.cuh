@@ -208,17 +208,6 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
                  : "memory");
 }
 
-// D[tmem] (+)= A[smem desc] . B[smem desc]^T, bf16 x bf16 -> fp32, issued by one thread.
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                          uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
 // Arrives on `bar` when every tcgen05.mma issued so far by this thread is done.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
@@ -330,7 +319,6 @@ __device__ __forceinline__ uint32_t make_idesc2(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
 }
 
-
 #if defined(MOE_B200_TEST_AIDS) && defined(TC5_TRACE)
 // Test-aids builds only (-DMOE_B200_TEST_AIDS -DTC5_TRACE=<MODE>): SM-clock timestamps of the
 // pipeline hand-offs of CTA 0.
@@ -344,7 +332,6 @@ __device__ long long g_trace[TRACE_STEPS * TRACE_SLOTS];
 #else
 #define TRACE(step, slot) do { } while (0)
 #endif
-#define TRACE_D(step, slot) TRACE(step, slot)
 
 #define RING_ADVANCE(s, ph, depth) \
     do {                           \
